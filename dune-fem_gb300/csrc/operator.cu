@@ -22,6 +22,9 @@ int dg_const_launch_f64(const DgArgsT<double>&, const DgConstTablesT<double>&, i
                         double* ucopy = nullptr);
 int dg_const_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, float*, int, cudaStream_t,
                         float* ucopy = nullptr);
+bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out);
+int dg_fixed_launch(const DgArgsT<double>&, const DgConstTablesT<double>&, const FxTables&, int n, int z0, int z1,
+                    cudaStream_t);
 int dg_cell_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t);
 bool dg_cell_supported(int n);
 int dg_kappa_points_f64(const double*, double*, double*, long long, const DgTablesT<double>&, int, int, cudaStream_t);
@@ -215,6 +218,12 @@ int dg_apply(const gbfem_operator_s* op, const void* u, void* w, cudaStream_t s,
   return GBFEM_OK;
 }
 
+// u (which may be page-locked host memory) to the device copy the apply reads
+__global__ void k_copy_dofs(long long n, const double* __restrict__ u, double* __restrict__ v) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    v[i] = __ldg(u + i);
+}
+
 static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, cudaStream_t s, int unit_mode,
                            void* blocks, long long cell_begin, long long cell_count, int phase, void* ucopy) {
   if (op->precision == GBFEM_F64) {
@@ -229,6 +238,21 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
     if (unit_mode == 0 && op->coefficient_space) {
       DgConstTablesT<double> ct = op->ctab64;
       fill_line_operators(op, &ct);
+      // One kernel over whole z-planes where the coefficients fit the fixed
+      // point (fx_make_tables).  It has no trace pass: phase 1 only copies.
+      // 64^3 Q3: 319 us against 822 for the two FP64-pipe kernels, which stay
+      // for a kappa per cell and refused coefficients.
+      const long long plane = (long long)a.nc[0] * a.nc[1];
+      const long long count = cell_count > 0 ? cell_count : op->ncells - cell_begin;
+      if (op->fixed && cell_begin % plane == 0 && count % plane == 0) {
+        if ((phase & 1) && ucopy) {
+          const long long n0 = cell_begin * op->nloc, nn = count * op->nloc;
+          k_copy_dofs<<<stream_grid(nn), 256, 0, s>>>(nn, a.u + n0, static_cast<double*>(ucopy) + n0);
+          GBFEM_CUDA_TRY(cudaGetLastError());
+        }
+        if (!(phase & 2)) return GBFEM_OK;
+        return dg_fixed_launch(a, ct, op->fx, op->n, int(cell_begin / plane), int((cell_begin + count) / plane), s);
+      }
       void* tb = nullptr;
       GBFEM_TRY(trace_buffer(op, &tb));
       return dg_const_launch_f64(a, ct, op->n, static_cast<double*>(tb), phase, s, static_cast<double*>(ucopy));
@@ -564,9 +588,9 @@ static int enqueue_copy_pipeline(gbfem_operator_s* op, HostPipe* p, const void* 
   // The closed form's trace pass of slab k runs on its own stream as soon as
   // slab k has arrived, so it fills the SMs left idle by the tail of the apply
   // of slab k-1 (a slab is only a wave or two of CTAs).  The apply of slab j
-  // reads the traces (or, for the quadrature kernel, the dofs) of slabs j-1,
+  // reads the traces (or, for the one-kernel forms, the dofs) of slabs j-1,
   // j and j+1, so it waits for slab j+1's traces (or arrival).
-  const bool traces = op->coefficient_space;
+  const bool traces = op->coefficient_space && !op->fixed;
   if (traces) {
     GBFEM_CUDA_TRY(cudaStreamWaitEvent(p->tr, p->start, 0));
     for (int k = 0; k < nchunks; ++k) {
@@ -603,7 +627,8 @@ static int enqueue_copy_pipeline(gbfem_operator_s* op, HostPipe* p, const void* 
 static int capture_copy_pipeline(gbfem_operator_s* op, HostPipe* p, const void* u_host, void* w_host, int nchunks,
                                  const std::vector<int>& zb) {
   drop_host_graph(p);
-  if (op->coefficient_space) {
+  const bool traces = op->coefficient_space && !op->fixed;
+  if (traces) {
     void* tb = nullptr;
     GBFEM_TRY(trace_buffer(op, &tb));
   }
@@ -611,7 +636,7 @@ static int capture_copy_pipeline(gbfem_operator_s* op, HostPipe* p, const void* 
   int rc = enqueue_copy_pipeline(op, p, u_host, w_host, zb, p->in);
   if (rc == GBFEM_OK) {
     // join every forked stream back into the origin
-    cudaStream_t forked[3] = {p->comp, p->out, op->coefficient_space ? p->tr : nullptr};
+    cudaStream_t forked[3] = {p->comp, p->out, traces ? p->tr : nullptr};
     for (int i = 0; i < 3 && rc == GBFEM_OK; ++i) {
       if (!forked[i]) continue;
       cudaError_t e = cudaEventRecord(p->join[i], forked[i]);
@@ -730,6 +755,7 @@ int gbfem_dg_operator_create(const gbfem_dg_desc* desc, gbfem_operator* out) {
   }
   op->coefficient_space = desc->kappa == nullptr && desc->algorithm != GBFEM_ALGO_QUADRATURE;
   op->two_kernel_f32 = desc->algorithm == GBFEM_ALGO_TRACE_PASS;
+  op->fixed = op->precision == GBFEM_F64 && op->coefficient_space && fx_make_tables(op->dg, op->n, &op->fx);
   const int rc = dg_kappa_cache(op);
   if (rc) {
     gbfem_operator_destroy(op);

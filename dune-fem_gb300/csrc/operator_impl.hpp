@@ -4,6 +4,7 @@
 
 #include "../../include/gbfem.h"
 #include "dg_const_kernel.cuh"
+#include "dg_fixed_tables.hpp"
 #include "dg_kernel.cuh"
 
 namespace gbfem {
@@ -56,6 +57,8 @@ struct gbfem_operator_s {
   gbfem::DgConstTablesT<float> ctab32{};
   bool coefficient_space = false;  // constant-coefficient closed form (exact quadrature)
   bool two_kernel_f32 = false;     // FP32 closed form: trace pass + apply even where one kernel applies
+  bool fixed = false;              // FP64 closed form in one kernel on the integer pipes (fx)
+  gbfem::FxTables fx{};
   double cK1[gbfem::kDgMaxN * gbfem::kDgMaxN] = {};  // 1-D stiffness int L_i' L_j'
   double cD1[gbfem::kDgMaxN * gbfem::kDgMaxN] = {};  // 1-D advection int L_i' L_j
   gbfem::Q1Element q1{};

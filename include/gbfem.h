@@ -90,12 +90,13 @@ typedef struct {
  * same integrals (orthonormal basis, affine cells, exact Gauss quadrature:
  * 1-D stiffness/advection matrices along lines, identity tangential face
  * mass), which equals the quadrature result up to rounding; otherwise the
- * sum-factorised quadrature kernel.  The closed form runs as a trace pass
- * into an operator-owned buffer followed by the apply, except FP32 with
- * p <= 3 over the whole grid, which is one kernel without the buffer.
+ * sum-factorised quadrature kernel.  The closed form is one kernel in FP64
+ * with a constant kappa (in 64-bit fixed point on the integer pipes) and in
+ * FP32 with p <= 3 over the whole grid; otherwise a trace pass into an
+ * operator-owned buffer followed by the apply.
  * GBFEM_ALGO_QUADRATURE always evaluates at the q^3 volume / q^2 face Gauss
- * points.  GBFEM_ALGO_TRACE_PASS is the closed form always in its trace-pass
- * form. */
+ * points.  GBFEM_ALGO_TRACE_PASS is the FP32 closed form always in its
+ * trace-pass form (in FP64 it is GBFEM_ALGO_AUTO). */
 #define GBFEM_ALGO_AUTO 0
 #define GBFEM_ALGO_QUADRATURE 1
 #define GBFEM_ALGO_TRACE_PASS 2
