@@ -1149,13 +1149,18 @@ static int fcg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_pa
 
 int solve_impl(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* f, void* u,
                gbfem_solver_info* info, cudaStream_t s) {
-  Ctx c;
-  GBFEM_TRY(c.setup(op->precision, op->ndofs, s));
   *info = gbfem_solver_info{};
   const auto t0 = std::chrono::steady_clock::now();
   int rc;
   if (prm.error_measure < GBFEM_TOL_ABSOLUTE || prm.error_measure > GBFEM_TOL_RELATIVE_RESIDUAL)
     return set_error(GBFEM_ERR_INVALID, "gbfem_solve: unknown error measure");
+  if (prm.method == GBFEM_SOLVER_CG && q1_cg_takes(op, pc, prm)) {
+    rc = q1_cg(op, pc, prm, f, u, s, info);
+    info->time_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    return rc;
+  }
+  Ctx c;
+  GBFEM_TRY(c.setup(op->precision, op->ndofs, s));
   // the other methods already stop on the unpreconditioned residual
   gbfem_solver_params pr = prm;
   if (prm.method != GBFEM_SOLVER_CG && pr.error_measure == GBFEM_TOL_RELATIVE_RESIDUAL)

@@ -19,6 +19,11 @@ int sb_tc_setup(struct ::gbfem_preconditioner_s* pc, const std::vector<int>& til
 int sb_tc_apply(const struct ::gbfem_preconditioner_s* pc, const float* kcell, const float* r, float* z,
                 cudaStream_t s);
 
+// the Q1 operator's CG in one kernel (q1_cg.cu), for the solves it takes
+bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
+int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
+          cudaStream_t s, gbfem_solver_info* info);
+
 }  // namespace gbfem
 
 struct gbfem_preconditioner_s {
