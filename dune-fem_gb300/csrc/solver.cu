@@ -541,8 +541,8 @@ int precond_apply(const gbfem_preconditioner_s* pc, const void* r, void* z, cuda
         g.nc[d] = pc->sor_op->dg.grid.cells[d];
         g.per[d] = pc->sor_op->dg.grid.periodic[d];
       }
-      if (pc->sb_engine == GBFEM_SB_ENGINE_TENSOR && pc->sb_tc_tiles) {
-        return sb_tc_apply(pc, (const float*)pc->sor_op->dg.kappa_cell, (const float*)r, (float*)z, s);
+      if (pc->sb_fdm) {
+        return sb_fdm_apply(pc, (const float*)r, (float*)z, s);
       } else if (pc->sb_tiles) {
         // one CTA per SM over a contiguous range of quads: the inverse and
         // two residual tiles per group, 192 KB at nb = 125
@@ -1327,11 +1327,7 @@ int gbfem_preconditioner_scaled_block_jacobi_create(gbfem_operator op, gbfem_pre
 
 int gbfem_preconditioner_status(gbfem_preconditioner pc, int* status) {
   if (!pc || !status) return set_error(GBFEM_ERR_INVALID, "gbfem_preconditioner_status: null argument");
-  *status = 0;
-  if (pc->sb_tc_status) {
-    GBFEM_CUDA_TRY(cudaDeviceSynchronize());
-    GBFEM_CUDA_TRY(cudaMemcpy(status, pc->sb_tc_status, sizeof(int), cudaMemcpyDeviceToHost));
-  }
+  *status = 0;  // no preconditioner kernel has a wait that can give up
   return GBFEM_OK;
 }
 
@@ -1344,6 +1340,22 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
   if (op->kind != OpKind::DG || !d.kappa_cell || op->precision != GBFEM_F32 || d.mass != 0.0 || op->nonlinear)
     return set_error(GBFEM_ERR_INVALID,
                      "scaled block Jacobi: needs an FP32 DG operator with kappa_cell, no mass, not nonlinear");
+  if (engine == GBFEM_SB_ENGINE_TENSOR) {
+    auto* pc = new (std::nothrow) gbfem_preconditioner_s();
+    if (!pc) return set_error(GBFEM_ERR_INVALID, "out of host memory");
+    pc->kind = PcKind::ScaledBlock;
+    pc->precision = GBFEM_F32;
+    pc->n = op->ndofs;
+    pc->nloc = op->nloc;
+    pc->sor_op = op;
+    const int rc = sb_fdm_setup(pc);
+    if (rc) {
+      gbfem_preconditioner_destroy(pc);
+      return rc;
+    }
+    *out = pc;
+    return GBFEM_OK;
+  }
   // the kappa = 1 operator on a grid with one cell per boundary type, same cell size
   gbfem_dg_desc t = d;
   t.kappa = nullptr;
@@ -1368,7 +1380,6 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
     return set_error(GBFEM_ERR_INVALID, "out of host memory");
   }
   pc->kind = PcKind::ScaledBlock;
-  pc->sb_engine = engine;
   pc->precision = GBFEM_F32;
   pc->n = op->ndofs;
   pc->nloc = op->nloc;
@@ -1422,13 +1433,6 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
       return set_cuda_error(e, "scaled block Jacobi: tiles");
     }
     pc->sb_ntiles = (long long)(tiles.size() / 3);
-    if (engine == GBFEM_SB_ENGINE_TENSOR) {
-      const int rc = sb_tc_setup(pc, tiles, op->nloc, 0);
-      if (rc) {
-        gbfem_preconditioner_destroy(pc);
-        return rc;
-      }
-    }
   }
   *out = pc;
   return GBFEM_OK;
@@ -1451,9 +1455,7 @@ int gbfem_preconditioner_destroy(gbfem_preconditioner pc) {
   if (pc->scales) cudaFree(pc->scales);
   if (pc->sor_cells) cudaFree(pc->sor_cells);
   if (pc->sb_tiles) cudaFree(pc->sb_tiles);
-  if (pc->sb_tc_tiles) cudaFree(pc->sb_tc_tiles);
-  if (pc->sb_tc_img) cudaFree(pc->sb_tc_img);
-  if (pc->sb_tc_status) cudaFree(pc->sb_tc_status);
+  if (pc->sb_fdm) sb_fdm_destroy(pc->sb_fdm);
   if (pc->sor_tmp) cudaFree(pc->sor_tmp);
   if (pc->ext_destroy) pc->ext_destroy(pc->ext_ctx);
   delete pc;

@@ -13,12 +13,10 @@ enum class PcKind { Diagonal = 1, BlockJacobi = 2, External = 3, Sor = 4, Scaled
 int precond_apply(const struct ::gbfem_preconditioner_s* pc, const void* r, void* z, cudaStream_t s);
 // Jacobi / Gauss-Seidel / SOR / SSOR sweeps over an assembled operator (sor.cu)
 int sor_apply(const struct ::gbfem_preconditioner_s* pc, const void* r, void* z, cudaStream_t s);
-// scaled block Jacobi on the tensor cores (sb_tc.cu): set-up from the
-// (type, start, count) tiles, and the apply
-int sb_tc_setup(struct ::gbfem_preconditioner_s* pc, const std::vector<int>& tiles3, int nb, cudaStream_t s);
-int sb_tc_apply(const struct ::gbfem_preconditioner_s* pc, const float* kcell, const float* r, float* z,
-                cudaStream_t s);
-
+// scaled block Jacobi by fast diagonalisation (sb_fdm.cu)
+int sb_fdm_setup(struct ::gbfem_preconditioner_s* pc);
+int sb_fdm_apply(const struct ::gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s);
+void sb_fdm_destroy(void* tables);
 // the Q1 operator's CG in one kernel (q1_cg.cu), for the solves it takes
 bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
@@ -51,16 +49,9 @@ struct gbfem_preconditioner_s {
   int* sor_cells = nullptr;
   void* sor_tmp = nullptr;
   std::vector<long long> sor_level_offsets;
-  // ScaledBlock: sor_cells holds the cells sorted by boundary type; tiles of
+  // ScaledBlock by dense tiles: sor_cells holds the cells sorted by boundary type; tiles of
   // (type, start, count) into it
   int* sb_tiles = nullptr;
   long long sb_ntiles = 0;
-  // ScaledBlock on the tensor cores: tiles without padding, A_hi | A_lo
-  // images per type, the kernel's status word (1 = a wait timed out)
-  int sb_engine = GBFEM_SB_ENGINE_TENSOR;
-  int* sb_tc_tiles = nullptr;
-  int sb_tc_ntiles = 0;
-  int sb_tc_wide = 0;  // 64-cell tiles with K = 64 (blocks of up to 64 dofs)
-  void* sb_tc_img = nullptr;
-  int* sb_tc_status = nullptr;
+  void* sb_fdm = nullptr;  // ScaledBlock by fast diagonalisation: its tables (host)
 };

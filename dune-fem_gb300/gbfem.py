@@ -619,14 +619,15 @@ class Preconditioner:
     def scaled_block_jacobi(cls, op, engine="tensor"):
         """For an FP32 operator with kappa_cell (no mass): z_c = H_t^-1 r_c / kappa_c
         with the shared kappa = 1 blocks H_t of the cell's boundary type.
-        engine: "tensor" (tcgen05, 3xTF32) or "fma" for the tile products."""
+        engine: "tensor" (the tensor-product form, by fast diagonalisation) or
+        "fma" (products with the dense inverses)."""
         h = C.c_void_p()
         eng = {"tensor": 0, "fma": 1}[engine]
         check(lib().gbfem_preconditioner_scaled_block_jacobi_create_engine(op.handle, eng, C.byref(h)))
         return cls(h, F32, op)
 
     def status(self):
-        """0, or 1 if a bounded wait in the tensor-core kernel gave up."""
+        """0 (1 would be a bounded wait in a kernel that gave up)."""
         st = C.c_int()
         check(lib().gbfem_preconditioner_status(self.handle, C.byref(st)))
         return st.value

@@ -1,0 +1,31 @@
+"""The scaled shared-block Jacobi in its tensor-product form (fast
+diagonalisation) against dense FP64 inverses of the oracle's kappa = 1 blocks."""
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("cells,kw", [
+    ((1, 1, 1), dict()),                                     # both boundaries on every axis, less than one warp of cells
+    ((2, 1, 7), dict(upper=(1.0, 0.3, 2.0), diffusion=2.5)),  # no interior cell, anisotropic
+    ((9, 6, 5), dict(upper=(1.0, 0.25, 3.0), penalty=55.0)),
+    ((33, 4, 3), dict(periodic=(0, 1, 0))),                  # CTAs with and without boundary cells
+])
+def test_against_dense_inverse(gb, orc, order, cells, kw):
+    """Relative to the largest entry of each cell's result: FP32 rounding of r
+    in the eigenbasis (2^-24 a step, about 6 n steps of sums) divided by the
+    smallest eigenvalue, against |z| >= |r| / (largest eigenvalue) -- bounded
+    here by the blocks' own condition number: 40 2^-24 cond."""
+    nc, nloc = int(np.prod(cells)), (order + 1) ** 3
+    rng = np.random.default_rng(order)
+    kc = np.exp(rng.uniform(-2, 2, nc)).astype(np.float32)
+    r = rng.uniform(-1, 1, nc * nloc).astype(np.float32)
+    op = gb.DGOperator(cells, order, precision=gb.F32, kappa_cell=gb.DeviceArray.from_numpy(kc), **kw)
+    z = gb.DeviceArray(nc * nloc, gb.F32)
+    gb.Preconditioner.scaled_block_jacobi(op)(gb.DeviceArray.from_numpy(r), z)
+    blocks = orc.DGProblem(cells, order, **kw).block_diagonal(nthreads=4)
+    ref = np.linalg.solve(blocks, r.astype(np.float64).reshape(nc, nloc, 1))[..., 0] / kc[:, None]
+    err = np.max(np.abs(z.numpy().reshape(nc, nloc) - ref), axis=1) / np.max(np.abs(ref), axis=1)
+    assert np.all(err <= 40 * 2.0 ** -24 * np.linalg.cond(blocks))
+    assert np.sqrt(np.mean(err ** 2)) < 2e-5
