@@ -37,6 +37,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "cg_device.cuh"
 #include "dg_const_kernel.cuh"
 
 namespace gbfem {
@@ -313,9 +314,13 @@ __device__ __forceinline__ int cell_boundary_face(int r, int c0, int c1, const C
   return 2;
 }
 
-template <int N, bool ADV, bool KC>
+// DOT: the operator of a device-resident CG iteration (cg_device.cuh): nothing
+// once it has converged; otherwise also <u, w>, and alpha by the last CTA.
+template <int N, bool ADV, bool KC, bool DOT = false>
 __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_constant__ DgArgsT<float> args,
-                                                                  const __grid_constant__ DgConstTablesT<float> tabs) {
+                                                                  const __grid_constant__ DgConstTablesT<float> tabs,
+                                                                  double* __restrict__ partial, CgScalars* sc) {
+  if (DOT && !sc->active) return;
   constexpr int N2 = N * N, N3 = N2 * N;
   using S = CellSlots<N>;
   static_assert(!(KC && ADV), "cellwise kappa without advection");
@@ -417,7 +422,7 @@ __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_c
     }
   }
   __syncthreads();
-  if (!valid) return;
+  if (!DOT && !valid) return;
 
   // ---- 3. line operator + face expansion, one pass per axis ----------------------
   float w[N3];
@@ -480,19 +485,31 @@ __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_c
       }
     }
   };
-  line_pass(std::integral_constant<int, 0>());
-  line_pass(std::integral_constant<int, 1>());
-  line_pass(std::integral_constant<int, 2>());
+  DotAcc<float> acc;
+  if (valid) {
+    line_pass(std::integral_constant<int, 0>());
+    line_pass(std::integral_constant<int, 1>());
+    line_pass(std::integral_constant<int, 2>());
 
-  // ---- 4. store ------------------------------------------------------------------
-  float* dst = args.w + cell * N3;
-  if constexpr (N3 % 4 == 0) {
-    float4* d4 = reinterpret_cast<float4*>(dst);
+    // ---- 4. store ----------------------------------------------------------------
+    float* dst = args.w + cell * N3;
+    if constexpr (N3 % 4 == 0) {
+      float4* d4 = reinterpret_cast<float4*>(dst);
 #pragma unroll
-    for (int q = 0; q < N3 / 4; ++q) __stcs(d4 + q, make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]));
-  } else {
+      for (int q = 0; q < N3 / 4; ++q) __stcs(d4 + q, make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]));
+    } else {
 #pragma unroll
-    for (int q = 0; q < N3; ++q) __stcs(dst + q, w[q]);
+      for (int q = 0; q < N3; ++q) __stcs(dst + q, w[q]);
+    }
+    if (DOT) {
+#pragma unroll
+      for (int q = 0; q < N3; ++q) acc.add(u[q], w[q]);
+    }
+  }
+  if constexpr (DOT) {
+    if (!cg_deliver(cg_block_part(acc), partial, sc, 0)) return;
+    const double t = cg_sum_parts(partial, int(gridDim.x));
+    if (tid == 0) cg_set_alpha(sc, t);
   }
 }
 

@@ -12,6 +12,7 @@
 #include "dg_kernel.cuh"
 #include "gbfem_internal.cuh"
 #include "operator_impl.hpp"
+#include "solver_impl.hpp"
 #include "tables.hpp"
 
 namespace gbfem {
@@ -25,7 +26,10 @@ int dg_const_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int
 bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out);
 int dg_fixed_launch(const DgArgsT<double>&, const DgConstTablesT<double>&, const FxTables&, int n, int z0, int z1,
                     cudaStream_t);
-int dg_cell_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t);
+struct CgScalars;
+int dg_cell_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t, double* partial = nullptr,
+                       CgScalars* sc = nullptr);
+long long dg_cell_blocks(const int* nc);
 bool dg_cell_supported(int n);
 int dg_kappa_points_f64(const double*, double*, double*, long long, const DgTablesT<double>&, int, int, cudaStream_t);
 int dg_kappa_points_f32(const float*, float*, float*, long long, const DgTablesT<float>&, int, int, cudaStream_t);
@@ -282,6 +286,23 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
     }
     return dg_launch_f32(a, op->tab32, op->n, op->q, op->dg.kappa != nullptr, s);
   }
+}
+
+// The device-resident CG's operator: the one-kernel FP32 closed form, which has a
+// cell's dofs and results in one thread's registers, with <q, h> in its end.
+long long cg_apply_dot_parts(const gbfem_operator_s* op) {
+  const bool cell = op->kind == OpKind::DG && op->precision == GBFEM_F32 && op->coefficient_space && !op->form &&
+                    !op->nonlinear && !op->jac_points && dg_cell_supported(op->n) && !op->two_kernel_f32;
+  return cell ? dg_cell_blocks(op->dg.grid.cells) : 0;
+}
+int cg_apply_dot(const gbfem_operator_s* op, const void* q, void* h, double* partial, CgScalars* sc, cudaStream_t s) {
+  DgArgsT<float> a;
+  fill_dg_args(op, &a);
+  a.u = static_cast<const float*>(q);
+  a.w = static_cast<float*>(h);
+  DgConstTablesT<float> ct = op->ctab32;
+  fill_line_operators(op, &ct);
+  return dg_cell_launch_f32(a, ct, op->n, s, partial, sc);
 }
 
 // ---- continuous Q1 (2-D) ---------------------------------------------------

@@ -25,6 +25,7 @@
 #include <cmath>
 #include <new>
 
+#include "cg_device.cuh"
 #include "gbfem_internal.cuh"
 #include "operator_impl.hpp"
 #include "solver_impl.hpp"
@@ -38,9 +39,15 @@ struct SbFdmTables {
   float L[3][4][kDgMaxN];
 };
 
+// CG: one iteration's end (cg_device.cuh).  r is p, updated to p - alpha h before
+// the preconditioner takes it; x += alpha q; then <p, z> and the scalars.
 struct SbFdmArgs {
   const float *kcell, *r;
   float* z;
+  const float *q, *h;
+  float *x, *p;
+  double* partial;
+  CgScalars* sc;
   long long ncells;
   int nc[3], periodic[3];
 };
@@ -78,7 +85,7 @@ __device__ __forceinline__ void sb_plane(float (&x)[N * N], const float* __restr
   }
 }
 
-template <int N>
+template <int N, bool CG>
 __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ SbFdmArgs g,
                                                         const __grid_constant__ SbFdmTables tabs) {
   using S = SbFdm<N>;
@@ -87,6 +94,8 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   __shared__ float sV[3 * 4 * N2];
   __shared__ float sL[3 * 4 * N];
   __shared__ float sInv[N3];  // 1 / (Lx + Ly + Lz) of an interior cell, [i0][i1][i2]
+  if (CG && !g.sc->active) return;
+  const float alpha = CG ? g.sc->alpha_f : 0.f, minus = -alpha;
   const int tid = threadIdx.x;
   const long long c0 = (long long)blockIdx.x * S::CPB;
   const int ncell = int(g.ncells - c0 < S::CPB ? g.ncells - c0 : S::CPB);
@@ -100,19 +109,53 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   const float* rg = g.r + c0 * N3;
   float* zg = g.z + c0 * N3;
   const int total = ncell * N3;
-  const bool wide = ((reinterpret_cast<uintptr_t>(rg) | reinterpret_cast<uintptr_t>(zg)) & 15) == 0 && total % 4 == 0;
+  const long long e0 = c0 * N3;
+  uintptr_t at = reinterpret_cast<uintptr_t>(rg) | reinterpret_cast<uintptr_t>(zg);
+  if (CG) at |= reinterpret_cast<uintptr_t>(g.q + e0) | reinterpret_cast<uintptr_t>(g.h + e0) |
+                reinterpret_cast<uintptr_t>(g.x + e0);
+  const bool wide = (at & 15) == 0 && total % 4 == 0;
   auto place = [](int e) { return N2 == PL ? e : (e / N2) * PL + e % N2; };
   constexpr int K4 = (N2 + 3) / 4;
+  float4 t[K4];  // CG: this thread's p, for <p, z>
   if (wide) {
-    float4 t[K4];
 #pragma unroll
     for (int j = 0; j < K4; ++j)
-      if (4 * (tid + j * T) < total) t[j] = __ldg(reinterpret_cast<const float4*>(rg) + tid + j * T);
+      if (4 * (tid + j * T) < total)
+        t[j] = CG ? reinterpret_cast<const float4*>(rg)[tid + j * T] : __ldg(reinterpret_cast<const float4*>(rg) + tid + j * T);
+    if constexpr (CG) {
+#pragma unroll
+      for (int j = 0; j < K4; ++j) {
+        const int v = tid + j * T;
+        if (4 * v < total) {
+          const float4 h = __ldg(reinterpret_cast<const float4*>(g.h + e0) + v);
+          const float4 q = __ldg(reinterpret_cast<const float4*>(g.q + e0) + v);
+          float4 x = reinterpret_cast<const float4*>(g.x + e0)[v];
+          x.x = alpha * q.x + x.x;
+          x.y = alpha * q.y + x.y;
+          x.z = alpha * q.z + x.z;
+          x.w = alpha * q.w + x.w;
+          reinterpret_cast<float4*>(g.x + e0)[v] = x;
+          t[j].x = minus * h.x + t[j].x;
+          t[j].y = minus * h.y + t[j].y;
+          t[j].z = minus * h.z + t[j].z;
+          t[j].w = minus * h.w + t[j].w;
+          reinterpret_cast<float4*>(g.p + e0)[v] = t[j];
+        }
+      }
+    }
 #pragma unroll
     for (int j = 0; j < K4; ++j)
       if (4 * (tid + j * T) < total) *reinterpret_cast<float4*>(buf + place(4 * (tid + j * T))) = t[j];
   } else {
-    for (int e = tid; e < total; e += T) buf[place(e)] = __ldg(rg + e);
+    for (int e = tid; e < total; e += T) {
+      float v = CG ? rg[e] : __ldg(rg + e);
+      if constexpr (CG) {
+        g.x[e0 + e] = alpha * g.q[e0 + e] + g.x[e0 + e];
+        v = minus * g.h[e0 + e] + v;
+        g.p[e0 + e] = v;
+      }
+      buf[place(e)] = v;
+    }
   }
   // this thread's cell and its type on each axis
   const int lc = tid / N, i = tid - lc * N;
@@ -195,13 +238,31 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   else sb_plane<N, 1, false>(x, sV + (8 + type[2]) * N2);
   write_plane();
   __syncthreads();
+  DotAcc<float> acc;
   if (wide) {
 #pragma unroll
     for (int j = 0; j < K4; ++j)
-      if (4 * (tid + j * T) < total)
-        reinterpret_cast<float4*>(zg)[tid + j * T] = *reinterpret_cast<const float4*>(buf + place(4 * (tid + j * T)));
+      if (4 * (tid + j * T) < total) {
+        const float4 v = *reinterpret_cast<const float4*>(buf + place(4 * (tid + j * T)));
+        reinterpret_cast<float4*>(zg)[tid + j * T] = v;
+        if (CG) {
+          acc.add(t[j].x, v.x);
+          acc.add(t[j].y, v.y);
+          acc.add(t[j].z, v.z);
+          acc.add(t[j].w, v.w);
+        }
+      }
   } else {
-    for (int e = tid; e < total; e += T) zg[e] = buf[place(e)];
+    for (int e = tid; e < total; e += T) {
+      const float v = buf[place(e)];
+      zg[e] = v;
+      if (CG) acc.add(g.p[e0 + e], v);
+    }
+  }
+  if constexpr (CG) {
+    if (!cg_deliver(cg_block_part(acc), g.partial, g.sc, 1)) return;
+    const double sum = cg_sum_parts(g.partial, int(gridDim.x));
+    if (tid == 0) cg_set_end(g.sc, sum);
   }
 }
 
@@ -288,17 +349,15 @@ static int sb_fdm_launch(const SbFdmArgs& a, const SbFdmTables& t, cudaStream_t 
   const long long grid = (a.ncells + S::CPB - 1) / S::CPB;
   if (grid <= 0) return GBFEM_OK;
   if (grid > 2147483647LL) return set_error(GBFEM_ERR_INVALID, "scaled block Jacobi: grid too large");
-  k_sb_fdm<N><<<unsigned(grid), S::T, 0, s>>>(a, t);
+  if (a.sc) k_sb_fdm<N, true><<<unsigned(grid), S::T, 0, s>>>(a, t);
+  else k_sb_fdm<N, false><<<unsigned(grid), S::T, 0, s>>>(a, t);
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
 
-int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s) {
+static int sb_fdm_run(const gbfem_preconditioner_s* pc, SbFdmArgs& a, cudaStream_t s) {
   const gbfem_operator_s* op = pc->sor_op;
-  SbFdmArgs a{};
   a.kcell = static_cast<const float*>(op->dg.kappa_cell);
-  a.r = r;
-  a.z = z;
   a.ncells = op->ncells;
   for (int d = 0; d < 3; ++d) {
     a.nc[d] = op->dg.grid.cells[d];
@@ -312,6 +371,34 @@ int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cud
     case 5: return sb_fdm_launch<5>(a, t, s);
   }
   return set_error(GBFEM_ERR_NOT_IMPLEMENTED, "scaled block Jacobi: unsupported order");
+}
+
+int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s) {
+  SbFdmArgs a{};
+  a.r = r;
+  a.z = z;
+  return sb_fdm_run(pc, a, s);
+}
+
+long long sb_fdm_cg_parts(const gbfem_preconditioner_s* pc) {
+  if (pc->kind != PcKind::ScaledBlock || !pc->sb_fdm) return 0;
+  const int n = pc->sor_op->n;
+  const int cpb = n == 2 ? SbFdm<2>::CPB : (n == 3 ? SbFdm<3>::CPB : (n == 4 ? SbFdm<4>::CPB : SbFdm<5>::CPB));
+  return (pc->sor_op->ncells + cpb - 1) / cpb;
+}
+
+int sb_fdm_cg(const gbfem_preconditioner_s* pc, const void* q, const void* h, void* x, void* p, void* s_out,
+              double* partial, CgScalars* sc, cudaStream_t s) {
+  SbFdmArgs a{};
+  a.r = static_cast<const float*>(p);
+  a.z = static_cast<float*>(s_out);
+  a.q = static_cast<const float*>(q);
+  a.h = static_cast<const float*>(h);
+  a.x = static_cast<float*>(x);
+  a.p = static_cast<float*>(p);
+  a.partial = partial;
+  a.sc = sc;
+  return sb_fdm_run(pc, a, s);
 }
 
 }  // namespace gbfem

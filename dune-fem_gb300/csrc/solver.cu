@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "blas.cuh"
+#include "cg_device.cuh"
 #include "gbfem_internal.cuh"
 #include "operator_impl.hpp"
 #include "solver_impl.hpp"
@@ -647,73 +648,101 @@ static int cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_par
 
 // ------------------------------------------------ CG, device-resident loop ---
 // The same statements as cg() above, with the Krylov scalars in device memory
-// (written by single-thread kernels) and the vector updates predicated on an
-// "active" flag, so chunks of `chunk` iterations can be captured once into a
-// CUDA graph and relaunched; the host reads the convergence flag once per
-// chunk instead of synchronising on every scalar product.  Divisions and
-// updates are the host loop's, so the iterates are identical.
-enum { DS_RES = 0, DS_PREV, DS_QH, DS_NEW, DS_ALPHA, DS_BETA, DS_TOL, DS_ACTIVE, DS_DIR, DS_CONV, DS_IT, DS_MAX,
-       DS_STATUS, DS_N };
+// (cg_device.cuh) and every kernel of an iteration skipped once it has
+// converged, so chunks of `chunk` iterations can be captured once into a CUDA
+// graph and relaunched; the host reads the convergence flag once per chunk
+// instead of synchronising on every scalar product.  The scalar products end in
+// their last CTA, which also does the scalar statement that follows (alpha; the
+// end of the iteration and beta): no single-CTA kernels in between.  Divisions
+// and updates are the host loop's, so the iterates are identical -- except with
+// the scaled block Jacobi, whose fused kernels sum in their own order.
 
-// begin of an iteration + direction update (q = s + beta q with a
-// preconditioner, p = beta p - r without): every thread derives the flags and
-// beta itself from the fields no kernel of this launch writes; thread 0
-// publishes them for the later kernels.
+// q = s + beta q with a preconditioner, p = beta p - r without
 template <typename T>
-__global__ void k_cg_begin_dir(long long n, double a, const T* __restrict__ x, T* __restrict__ y, double* ds) {
-  const bool conv = ds[DS_CONV] != 0.0;
-  const bool dir = !conv && ds[DS_IT] > 0.0;
-  const double beta = dir ? ds[DS_RES] / ds[DS_PREV] : 0.0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ds[DS_ACTIVE] = conv ? 0.0 : 1.0;
-    ds[DS_DIR] = dir ? 1.0 : 0.0;
-    ds[DS_BETA] = beta;
-  }
-  if (!dir) return;
-  const T b = T(beta);
+__global__ void k_cg_dir(long long n, T a, const T* __restrict__ x, T* __restrict__ y, const CgScalars* sc) {
+  if (!sc->active || !sc->dir) return;
+  const T b = cg_beta<T>(sc);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    y[i] = T(a) * x[i] + b * y[i];
+    y[i] = a * x[i] + b * y[i];
 }
-// pass 2 of <q, h>, then alpha = rho / <q, h>
-__global__ void __launch_bounds__(kRedThreads) k_cg_final_alpha(const double* __restrict__ partial, int np,
-                                                                double* ds) {
-  const double qh = dot_final_sum(partial, np);
-  if (threadIdx.x != 0) return;
-  ds[DS_QH] = qh;
-  if (ds[DS_ACTIVE] == 0.0) return;
-  const double alpha = ds[DS_RES] / qh;
-  if (!isfinite(alpha)) {
-    ds[DS_STATUS] = 1.0;
-    ds[DS_CONV] = 1.0;
-    ds[DS_ACTIVE] = 0.0;
-    return;
+// the same for FP32 in 16-byte accesses (n4 = n / 4)
+__global__ void k_cg_dir4(long long n4, float a, const float4* __restrict__ x, float4* __restrict__ y,
+                          const CgScalars* sc) {
+  if (!sc->active || !sc->dir) return;
+  const float b = sc->beta_f;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
+    const float4 u = __ldg(x + i);
+    float4 v = y[i];
+    v.x = a * u.x + b * v.x;
+    v.y = a * u.y + b * v.y;
+    v.z = a * u.z + b * v.z;
+    v.w = a * u.w + b * v.w;
+    y[i] = v;
   }
-  ds[DS_ALPHA] = alpha;
+}
+
+// gbfem_dot's order over a chunk, four loads ahead
+template <typename T>
+__device__ __forceinline__ void cg_dot_chunk(const T* __restrict__ x, const T* __restrict__ y, long long b0, long long b1,
+                                             DotAcc<T>& acc) {
+  long long i = b0 + threadIdx.x;
+  for (; i + 3 * kRedThreads < b1; i += 4 * kRedThreads) {
+    T u[4], v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      u[k] = x[i + k * kRedThreads];
+      v[k] = y[i + k * kRedThreads];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc.add(u[k], v[k]);
+  }
+  for (; i < b1; i += kRedThreads) acc.add(x[i], y[i]);
+}
+// the last CTA's sum in gbfem_dot's order (dot_final_sum)
+__device__ __forceinline__ double cg_final_sum(const double* partial, int np) {
+  double s = 0.0;
+  for (int i = threadIdx.x; i < np; i += kRedThreads) s += __ldcg(partial + i);
+  return block_sum(s);
+}
+
+// <x, y>, then alpha (STEP 0) or the end of the iteration (STEP 1)
+template <typename T, int STEP>
+__global__ void __launch_bounds__(kRedThreads) k_cg_dot(long long n, long long chunk, const T* __restrict__ x,
+                                                        const T* __restrict__ y, double* __restrict__ partial,
+                                                        CgScalars* sc) {
+  if (!sc->active) return;
+  const long long b0 = (long long)blockIdx.x * chunk;
+  const long long b1 = b0 + chunk < n ? b0 + chunk : n;
+  DotAcc<T> acc;
+  cg_dot_chunk(x, y, b0, b1, acc);
+  if (!cg_deliver(block_sum(acc.value()), partial, sc, STEP)) return;
+  const double t = cg_final_sum(partial, int(gridDim.x));
+  if (threadIdx.x == 0) {
+    if (STEP == 0) cg_set_alpha(sc, t);
+    else cg_set_end(sc, t);
+  }
 }
 // x += alpha q; v += sv alpha h (v = p, sv = -1 with the diagonal
-// preconditioner; v = r, sv = +1 without), if active; then, in the partition
-// of pass 1 of a dot product: PC 0 the partial of <r, r>, PC 1 s = dinv p and
-// the partial of <p, s>.
+// preconditioner; v = r, sv = +1 without); then, in the partition of pass 1 of
+// a dot product: PC 0 the partial of <r, r>, PC 1 s = dinv p and the partial of
+// <p, s>; then the end of the iteration.
 template <typename T, int PC>
 __global__ void __launch_bounds__(kRedThreads) k_cg_update_dot(long long n, long long chunk, const T* __restrict__ q,
                                                                const T* __restrict__ h, T* __restrict__ x,
-                                                               T* __restrict__ v, double sv,
-                                                               const T* __restrict__ dinv, T* __restrict__ sz,
-                                                               double* __restrict__ partial, const double* ds) {
-  const bool active = ds[DS_ACTIVE] != 0.0;
-  const T alpha = T(ds[DS_ALPHA]);
-  const T sa = T(sv * ds[DS_ALPHA]);
+                                                               T* __restrict__ v, T sv, const T* __restrict__ dinv,
+                                                               T* __restrict__ sz, double* __restrict__ partial,
+                                                               CgScalars* sc) {
+  if (!sc->active) return;
+  const T alpha = cg_alpha<T>(sc);
+  const T sa = sv * alpha;
   const long long b0 = (long long)blockIdx.x * chunk;
   long long b1 = b0 + chunk;
   if (b1 > n) b1 = n;
   DotAcc<T> acc;  // the order and arithmetic of dot_partial_kernel
   for (long long i = b0 + threadIdx.x; i < b1; i += kRedThreads) {
-    T vi = v[i];
-    if (active) {
-      x[i] = alpha * q[i] + T(1) * x[i];
-      vi = sa * h[i] + T(1) * vi;
-      v[i] = vi;
-    }
+    x[i] = alpha * q[i] + T(1) * x[i];
+    const T vi = sa * h[i] + T(1) * v[i];
+    v[i] = vi;
     if (PC == 1) {
       const T si = vi * dinv[i];
       sz[i] = si;
@@ -722,51 +751,64 @@ __global__ void __launch_bounds__(kRedThreads) k_cg_update_dot(long long n, long
       acc.add(vi, vi);
     }
   }
-  const double sum = block_sum(acc.value());
-  if (threadIdx.x == 0) partial[blockIdx.x] = sum;
+  if (!cg_deliver(block_sum(acc.value()), partial, sc, 1)) return;
+  const double t = cg_final_sum(partial, int(gridDim.x));
+  if (threadIdx.x == 0) cg_set_end(sc, t);
 }
-// x += alpha q; p -= alpha h, if active (a general preconditioner follows):
-// grid-stride, since no dot-product partition has to be kept
+// x += alpha q; p -= alpha h (a general preconditioner follows): grid-stride,
+// since no dot-product partition has to be kept
 template <typename T>
 __global__ void k_cg_update(long long n, const T* __restrict__ q, const T* __restrict__ h, T* __restrict__ x,
-                            T* __restrict__ v, double sv, const double* ds) {
-  if (ds[DS_ACTIVE] == 0.0) return;
-  const T alpha = T(ds[DS_ALPHA]);
-  const T sa = T(sv * ds[DS_ALPHA]);
+                            T* __restrict__ v, T sv, const CgScalars* sc) {
+  if (!sc->active) return;
+  const T alpha = cg_alpha<T>(sc);
+  const T sa = sv * alpha;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     x[i] = alpha * q[i] + T(1) * x[i];
     v[i] = sa * h[i] + T(1) * v[i];
   }
 }
-// pass 2 of the new rho, then the end of the iteration
-__global__ void __launch_bounds__(kRedThreads) k_cg_final_end(const double* __restrict__ partial, int np,
-                                                              double* ds) {
-  const double rho = dot_final_sum(partial, np);
-  if (threadIdx.x != 0) return;
-  ds[DS_NEW] = rho;
-  if (ds[DS_ACTIVE] == 0.0) return;
-  ds[DS_PREV] = ds[DS_RES];
-  ds[DS_RES] = ds[DS_NEW];
-  ds[DS_IT] += 1.0;
-  if (!(ds[DS_RES] > ds[DS_TOL]) || ds[DS_IT] >= ds[DS_MAX]) ds[DS_CONV] = 1.0;
-  if (!isfinite(ds[DS_RES])) {
-    ds[DS_STATUS] = 1.0;
-    ds[DS_CONV] = 1.0;
+
+// Work vectors, scalars and captured iterations of cg_device, for a caller that
+// solves with the same operator, preconditioner and vectors again (the inner
+// solves of one mixed solve).
+struct CgDeviceState {
+  Vecs tmp;
+  CgScalars* sc = nullptr;
+  double* partial = nullptr;
+  cudaStream_t st = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  ~CgDeviceState() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (st) cudaStreamDestroy(st);
+    if (partial) cudaFree(partial);
+    if (sc) cudaFree(sc);
   }
-}
+};
 
 static int cg_device(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b,
-                     void* x, Ctx& c, gbfem_solver_info* info) {
-  Vecs tmp;
-  GBFEM_TRY(tmp.alloc(pc ? 5 : 3, c.bytes()));
-  void* h = tmp[0];
-  void* r = tmp[1];
-  void* p = tmp[2];
-  void* s = pc ? tmp[3] : p;
-  void* q = pc ? tmp[4] : p;
-  double* ds = nullptr;
-  GBFEM_CUDA_TRY(cudaMalloc(&ds, sizeof(double) * DS_N));
-  struct Free { double* p; ~Free() { cudaFree(p); } } free_ds{ds};
+                     void* x, Ctx& c, gbfem_solver_info* info, CgDeviceState* keep) {
+  CgDeviceState own;
+  CgDeviceState& w = keep ? *keep : own;
+  const long long n = c.n;
+  const int np = dot_num_partials(n);
+  // fused kernels: the whole-grid FP32 closed form with <q, h>, and the update
+  // with the scaled block Jacobi and <p, s>
+  const bool fuse_apply = cg_apply_dot_parts(op) > 0;
+  const bool fuse_pc = pc && sb_fdm_cg_parts(pc) > 0;
+  if (!w.sc) {
+    GBFEM_TRY(w.tmp.alloc(pc ? 5 : 3, c.bytes()));
+    long long parts = np;
+    if (fuse_apply) parts = std::max<long long>(parts, cg_apply_dot_parts(op));
+    if (fuse_pc) parts = std::max<long long>(parts, sb_fdm_cg_parts(pc));
+    GBFEM_CUDA_TRY(cudaMalloc(&w.partial, sizeof(double) * size_t(parts)));
+    GBFEM_CUDA_TRY(cudaMalloc(&w.sc, sizeof(CgScalars)));
+  }
+  void* h = w.tmp[0];
+  void* r = w.tmp[1];
+  void* p = w.tmp[2];
+  void* s = pc ? w.tmp[3] : p;
+  void* q = pc ? w.tmp[4] : p;
   // set-up, as cg(): h = A x, r = h - b, p = b - h, q = s = P p
   GBFEM_TRY(op_apply(op, x, h, c));
   GBFEM_TRY(c.copy(h, r));
@@ -783,92 +825,102 @@ static int cg_device(gbfem_operator op, gbfem_preconditioner pc, const gbfem_sol
   const double tolerance = prm.tolerance * prm.tolerance *
                            (prm.error_measure == GBFEM_TOL_RELATIVE ? bb
                             : prm.error_measure == GBFEM_TOL_RESIDUAL_REDUCTION ? residual : 1.0);
-  double h0[DS_N] = {};
-  h0[DS_RES] = residual;
-  h0[DS_TOL] = tolerance;
-  h0[DS_MAX] = double(prm.max_iterations);
-  h0[DS_CONV] = (residual > tolerance && 0 < prm.max_iterations) ? 0.0 : 1.0;
-  if (!finite(residual) || !finite(tolerance)) { h0[DS_CONV] = 1.0; h0[DS_STATUS] = 1.0; }
-  GBFEM_CUDA_TRY(cudaMemcpyAsync(ds, h0, sizeof(h0), cudaMemcpyHostToDevice, c.s));
-  // one iteration, as a function of the stream
-  const long long n = c.n;
+  CgScalars h0{};
+  h0.res = residual;
+  h0.tol = tolerance;
+  h0.max_it = prm.max_iterations;
+  h0.conv = (residual > tolerance && 0 < prm.max_iterations) ? 0 : 1;
+  if (!finite(residual) || !finite(tolerance)) { h0.conv = 1; h0.status = 1; }
+  h0.active = h0.conv ? 0 : 1;
+  GBFEM_CUDA_TRY(cudaMemcpyAsync(w.sc, &h0, sizeof(h0), cudaMemcpyHostToDevice, c.s));
   const int g = stream_grid(n);
-  const int np = dot_num_partials(n);
   const long long dchunk = (n + np - 1) / np;
   const bool diag_pc = pc && pc->kind == PcKind::Diagonal;
-  // one iteration, as a function of the stream: 6 launches (plus the operator
-  // and a general preconditioner with its dot product)
+  CgScalars* const sc = w.sc;
+  double* const partial = w.partial;
+  // one iteration, as a function of the stream: direction, operator, <q, h>,
+  // update, preconditioner, <p, s> (three launches where both ends are fused)
   auto iteration = [&](cudaStream_t st) -> int {
-    if (c.prec == GBFEM_F64) {
-      if (pc) k_cg_begin_dir<double><<<g, 256, 0, st>>>(n, 1.0, (const double*)s, (double*)q, ds);
-      else k_cg_begin_dir<double><<<g, 256, 0, st>>>(n, -1.0, (const double*)r, (double*)p, ds);
+    const void* dx = pc ? s : r;
+    void* dy = pc ? q : p;
+    if (c.prec == GBFEM_F64)
+      k_cg_dir<double><<<g, 256, 0, st>>>(n, pc ? 1.0 : -1.0, (const double*)dx, (double*)dy, sc);
+    else if (n % 4 == 0)  // (work vectors are 256-byte aligned)
+      k_cg_dir4<<<stream_grid(n / 4), 256, 0, st>>>(n / 4, pc ? 1.f : -1.f, (const float4*)dx, (float4*)dy, sc);
+    else
+      k_cg_dir<float><<<g, 256, 0, st>>>(n, pc ? 1.f : -1.f, (const float*)dx, (float*)dy, sc);
+    if (fuse_apply) {
+      GBFEM_TRY(cg_apply_dot(op, q, h, partial, sc, st));
     } else {
-      if (pc) k_cg_begin_dir<float><<<g, 256, 0, st>>>(n, 1.0, (const float*)s, (float*)q, ds);
-      else k_cg_begin_dir<float><<<g, 256, 0, st>>>(n, -1.0, (const float*)r, (float*)p, ds);
+      GBFEM_TRY(gbfem_operator_apply(op, q, h, st));
+      if (c.prec == GBFEM_F64)
+        k_cg_dot<double, 0><<<np, kRedThreads, 0, st>>>(n, dchunk, (const double*)q, (const double*)h, partial, sc);
+      else
+        k_cg_dot<float, 0><<<np, kRedThreads, 0, st>>>(n, dchunk, (const float*)q, (const float*)h, partial, sc);
     }
-    GBFEM_TRY(gbfem_operator_apply(op, q, h, st));
-    int npp = 0;
-    GBFEM_TRY(dot_partial_device(c.prec, n, q, h, c.d_partial, &npp, st));
-    k_cg_final_alpha<<<1, kRedThreads, 0, st>>>(c.d_partial, np, ds);
+    if (fuse_pc) return sb_fdm_cg(pc, q, h, x, p, s, partial, sc, st);
     void* v = pc ? p : r;
-    const double sv = pc ? -1.0 : 1.0;
     const int mode = !pc ? 0 : (diag_pc ? 1 : 2);
-#define GBFEM_CG_UPDATE(TT, M)                                                                              \
-  k_cg_update_dot<TT, M><<<np, kRedThreads, 0, st>>>(n, dchunk, (const TT*)q, (const TT*)h, (TT*)x, (TT*)v, sv, \
-                                                     diag_pc ? (const TT*)pc->data : nullptr, (TT*)s, c.d_partial, ds)
+#define GBFEM_CG_UPDATE(TT, M)                                                                                 \
+  k_cg_update_dot<TT, M><<<np, kRedThreads, 0, st>>>(n, dchunk, (const TT*)q, (const TT*)h, (TT*)x, (TT*)v,    \
+                                                     TT(pc ? -1 : 1), diag_pc ? (const TT*)pc->data : nullptr, \
+                                                     (TT*)s, partial, sc)
     if (c.prec == GBFEM_F64) {
       if (mode == 0) GBFEM_CG_UPDATE(double, 0);
       else if (mode == 1) GBFEM_CG_UPDATE(double, 1);
-      else k_cg_update<double><<<g, 256, 0, st>>>(n, (const double*)q, (const double*)h, (double*)x, (double*)v, sv, ds);
+      else k_cg_update<double><<<g, 256, 0, st>>>(n, (const double*)q, (const double*)h, (double*)x, (double*)v, -1.0, sc);
     } else {
       if (mode == 0) GBFEM_CG_UPDATE(float, 0);
       else if (mode == 1) GBFEM_CG_UPDATE(float, 1);
-      else k_cg_update<float><<<g, 256, 0, st>>>(n, (const float*)q, (const float*)h, (float*)x, (float*)v, sv, ds);
+      else k_cg_update<float><<<g, 256, 0, st>>>(n, (const float*)q, (const float*)h, (float*)x, (float*)v, -1.f, sc);
     }
 #undef GBFEM_CG_UPDATE
     if (mode == 2) {
       GBFEM_TRY(precond_apply(pc, p, s, st));
-      GBFEM_TRY(dot_partial_device(c.prec, n, p, s, c.d_partial, &npp, st));
+      if (c.prec == GBFEM_F64)
+        k_cg_dot<double, 1><<<np, kRedThreads, 0, st>>>(n, dchunk, (const double*)p, (const double*)s, partial, sc);
+      else
+        k_cg_dot<float, 1><<<np, kRedThreads, 0, st>>>(n, dchunk, (const float*)p, (const float*)s, partial, sc);
     }
-    k_cg_final_end<<<1, kRedThreads, 0, st>>>(c.d_partial, np, ds);
     GBFEM_CUDA_TRY(cudaGetLastError());
     return GBFEM_OK;
   };
   // capture `chunk` iterations into a graph on a private stream
   const int chunk = prm.graph_chunk > 0 ? prm.graph_chunk : 16;
-  cudaStream_t st = nullptr;
-  GBFEM_CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  struct FreeStream { cudaStream_t s; ~FreeStream() { cudaStreamDestroy(s); } } free_st{st};
+  if (!w.st) GBFEM_CUDA_TRY(cudaStreamCreateWithFlags(&w.st, cudaStreamNonBlocking));
   GBFEM_CUDA_TRY(cudaStreamSynchronize(c.s));
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
-  GBFEM_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
-  int rc = GBFEM_OK;
-  for (int k = 0; k < chunk && rc == GBFEM_OK; ++k) rc = iteration(st);
-  cudaError_t e = cudaStreamEndCapture(st, &graph);
-  if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
-  if (e != cudaSuccess) return set_cuda_error(e, "cg graph capture");
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return set_cuda_error(e, "cg graph instantiate");
-  struct FreeExec { cudaGraphExec_t g; ~FreeExec() { cudaGraphExecDestroy(g); } } free_exec{exec};
-  double hs[DS_N];
+  if (!w.exec) {
+    cudaGraph_t graph = nullptr;
+    GBFEM_CUDA_TRY(cudaStreamBeginCapture(w.st, cudaStreamCaptureModeRelaxed));
+    int rc = GBFEM_OK;
+    for (int k = 0; k < chunk && rc == GBFEM_OK; ++k) rc = iteration(w.st);
+    cudaError_t e = cudaStreamEndCapture(w.st, &graph);
+    if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
+    if (e != cudaSuccess) return set_cuda_error(e, "cg graph capture");
+    e = cudaGraphInstantiate(&w.exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) {
+      w.exec = nullptr;
+      return set_cuda_error(e, "cg graph instantiate");
+    }
+  }
+  CgScalars hs;
   int launches = 0;
   while (true) {
-    GBFEM_CUDA_TRY(cudaMemcpyAsync(hs, ds, sizeof(hs), cudaMemcpyDeviceToHost, st));
-    GBFEM_CUDA_TRY(cudaStreamSynchronize(st));
-    if (hs[DS_CONV] != 0.0) break;
-    GBFEM_CUDA_TRY(cudaGraphLaunch(exec, st));
+    GBFEM_CUDA_TRY(cudaMemcpyAsync(&hs, w.sc, sizeof(hs), cudaMemcpyDeviceToHost, w.st));
+    GBFEM_CUDA_TRY(cudaStreamSynchronize(w.st));
+    if (hs.conv) break;
+    GBFEM_CUDA_TRY(cudaGraphLaunch(w.exec, w.st));
     ++launches;
-    if (prm.verbose) std::printf("gbfem CG (graph) it: %d : residual %.6e\n", int(hs[DS_IT]), std::sqrt(hs[DS_RES]));
+    if (prm.verbose) std::printf("gbfem CG (graph) it: %d : residual %.6e\n", hs.it, std::sqrt(hs.res));
   }
-  const int it = int(hs[DS_IT]);
-  if (hs[DS_STATUS] != 0.0) info->status = GBFEM_ERR_NONFINITE;
-  info->residual = std::sqrt(std::fabs(hs[DS_RES]));
+  const int it = hs.it;
+  if (hs.status) info->status = GBFEM_ERR_NONFINITE;
+  info->residual = std::sqrt(std::fabs(hs.res));
   info->iterations = it < prm.max_iterations ? it : -it;
   info->converged = (it < prm.max_iterations && info->status == GBFEM_OK) ? 1 : 0;
   // applies launched: the set-up's plus every captured iteration (the ones
-  // after convergence recompute unchanged vectors and are not counted in `it`)
+  // after convergence do nothing and are not counted in `it`)
   c.op_applies += chunk * launches + 1;
   c.pc_applies += pc ? chunk * launches + 1 : 0;
   return GBFEM_OK;
@@ -1148,7 +1200,7 @@ static int fcg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_pa
 }
 
 int solve_impl(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* f, void* u,
-               gbfem_solver_info* info, cudaStream_t s) {
+               gbfem_solver_info* info, cudaStream_t s, CgDeviceState* keep) {
   *info = gbfem_solver_info{};
   const auto t0 = std::chrono::steady_clock::now();
   int rc;
@@ -1172,7 +1224,7 @@ int solve_impl(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_pa
       // stop is on the unpreconditioned residual (host loop)
       rc = (pr.graph_chunk > 0 && !(pc && pc->kind == PcKind::External) &&
             pr.error_measure != GBFEM_TOL_RELATIVE_RESIDUAL)
-               ? cg_device(op, pc, pr, f, u, c, info)
+               ? cg_device(op, pc, pr, f, u, c, info, keep)
                : cg(op, pc, pr, f, u, c, info);
       break;
     case GBFEM_SOLVER_GMRES: rc = gmres(op, pc, pr, f, u, c, info, false); break;
@@ -1468,7 +1520,7 @@ int gbfem_solve(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_p
   if (pc && pc->precision != op->precision)
     return set_error(GBFEM_ERR_INVALID, "gbfem_solve: preconditioner and operator precisions differ");
   if (pc && pc->n != op->ndofs) return set_error(GBFEM_ERR_INVALID, "gbfem_solve: preconditioner size mismatch");
-  return solve_impl(op, pc, *prm, f, u, info, nullptr);
+  return solve_impl(op, pc, *prm, f, u, info, nullptr, nullptr);
 }
 
 }  // extern "C"
@@ -1487,6 +1539,7 @@ struct InnerSolvePc {
   void* d32;
   long long inner_total = 0;
   int op_applies = 0, pc_applies = 0;
+  CgDeviceState cg;  // kept over the inner solves
 };
 
 static int inner_solve_apply(void* ctx, const void* r, void* z, cudaStream_t s) {
@@ -1502,7 +1555,7 @@ static int inner_solve_apply(void* ctx, const void* r, void* z, cudaStream_t s) 
   GBFEM_TRY(gbfem_scal(GBFEM_F32, x->n, 1.0 / rn, x->r32, s));
   GBFEM_CUDA_TRY(cudaMemsetAsync(x->d32, 0, size_t(x->n) * 4, s));
   gbfem_solver_info ii{};
-  GBFEM_TRY(solve_impl(x->op32, x->pc32, x->ip, x->r32, x->d32, &ii, s));
+  GBFEM_TRY(solve_impl(x->op32, x->pc32, x->ip, x->r32, x->d32, &ii, s, &x->cg));
   x->inner_total += ii.iterations >= 0 ? ii.iterations : -ii.iterations;
   x->op_applies += ii.operator_applies;
   x->pc_applies += ii.preconditioner_applies;
@@ -1575,7 +1628,7 @@ int gbfem_solve_mixed(gbfem_operator op64, gbfem_operator op32, gbfem_preconditi
       if (remaining <= 0) break;
       op.max_iterations = remaining < op.restart ? remaining : op.restart;
       oi = gbfem_solver_info{};
-      const int rc = solve_impl(op64, &px, op, f, u, &oi, nullptr);
+      const int rc = solve_impl(op64, &px, op, f, u, &oi, nullptr, nullptr);
       if (rc) {
         px.ext_ctx = nullptr;
         return rc;
@@ -1612,6 +1665,7 @@ int gbfem_solve_mixed(gbfem_operator op64, gbfem_operator op32, gbfem_preconditi
     info->preconditioner_applies = ctx.pc_applies;
     return GBFEM_OK;
   }
+  CgDeviceState inner_cg;  // kept over the inner solves
   for (outer = 0; outer <= prm->max_outer; ++outer) {
     GBFEM_TRY(op_apply(op64, u, r, c64));
     GBFEM_TRY(c64.axpby(1.0, f, -1.0, r));  // r = f - A u
@@ -1633,7 +1687,7 @@ int gbfem_solve_mixed(gbfem_operator op64, gbfem_operator op32, gbfem_preconditi
     GBFEM_TRY(c32.scal(1.0 / rn, r32));
     GBFEM_TRY(c32.clear(d32));
     gbfem_solver_info ii{};
-    GBFEM_TRY(solve_impl(op32, pc32, ip, r32, d32, &ii, nullptr));
+    GBFEM_TRY(solve_impl(op32, pc32, ip, r32, d32, &ii, nullptr, &inner_cg));
     inner_total += ii.iterations >= 0 ? ii.iterations : -ii.iterations;
     c64.op_applies += ii.operator_applies;
     c64.pc_applies += ii.preconditioner_applies;

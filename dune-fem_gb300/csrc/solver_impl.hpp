@@ -17,6 +17,17 @@ int sor_apply(const struct ::gbfem_preconditioner_s* pc, const void* r, void* z,
 int sb_fdm_setup(struct ::gbfem_preconditioner_s* pc);
 int sb_fdm_apply(const struct ::gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s);
 void sb_fdm_destroy(void* tables);
+struct CgScalars;
+// the fused kernels of the device-resident CG: x += alpha q, p -= alpha h, s = P p,
+// <p, s> and the end of the iteration; the number of CTAs (parts), 0 where the
+// preconditioner is another one
+long long sb_fdm_cg_parts(const struct ::gbfem_preconditioner_s* pc);
+int sb_fdm_cg(const struct ::gbfem_preconditioner_s* pc, const void* q, const void* h, void* x, void* p, void* s_out,
+              double* partial, CgScalars* sc, cudaStream_t s);
+// h = A q, <q, h> and alpha; 0 parts where the operator has no such kernel
+long long cg_apply_dot_parts(const struct ::gbfem_operator_s* op);
+int cg_apply_dot(const struct ::gbfem_operator_s* op, const void* q, void* h, double* partial, CgScalars* sc,
+                 cudaStream_t s);
 // the Q1 operator's CG in one kernel (q1_cg.cu), for the solves it takes
 bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
