@@ -180,13 +180,13 @@ struct DgSmem {
   static constexpr int TOTAL = TAB + CPB * PER_CELL;
 };
 
+// The apply of the CPB cells (virtual cells in unit mode) from v0 on, by all
+// threads of the CTA; sm: S::TOTAL elements.
 template <typename T, int N, int Q, bool KAPPA, int CPB>
-__global__ void __launch_bounds__(256) dg_apply_kernel(const DgArgsT<T> args,
-                                                       const __grid_constant__ DgTablesT<T> tabs) {
+__device__ __forceinline__ void dg_apply_cells(const DgArgsT<T>& args, const DgTablesT<T>& tabs, T* sm,
+                                               long long v0) {
   using S = DgSmem<N, Q, KAPPA, CPB>;
   constexpr int N3 = S::N3, Q3 = S::Q3, N2 = S::N2, Q2 = S::Q2, MA = S::MA;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sm = reinterpret_cast<T*>(smem_raw);
   T* sB = sm;
   T* sDc = sB + kDgMaxQ * kDgMaxN;
   T* sw = sDc + kDgMaxQ * kDgMaxQ;
@@ -211,7 +211,6 @@ __global__ void __launch_bounds__(256) dg_apply_kernel(const DgArgsT<T> args,
   const long long ucount = args.cell_count > 0 ? args.cell_count : ncells;
   const int vper = args.unit_mode == 3 ? 6 * N3 : (args.unit_mode ? N3 : 1);
   const long long nvirt = (args.cell_begin + ucount) * vper;
-  const long long v0 = (long long)blockIdx.x * CPB + args.cell_begin * vper;
   if (v0 >= nvirt) return;
 
   // ---- load own dofs --------------------------------------------------------
@@ -466,6 +465,15 @@ __global__ void __launch_bounds__(256) dg_apply_kernel(const DgArgsT<T> args,
       __stcs(args.w + v * N3 + i, sr[e]);
     }
   }
+}
+
+template <typename T, int N, int Q, bool KAPPA, int CPB>
+__global__ void __launch_bounds__(256) dg_apply_kernel(const DgArgsT<T> args,
+                                                       const __grid_constant__ DgTablesT<T> tabs) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int vper = args.unit_mode == 3 ? 6 * N * N * N : (args.unit_mode ? N * N * N : 1);
+  dg_apply_cells<T, N, Q, KAPPA, CPB>(args, tabs, reinterpret_cast<T*>(smem_raw),
+                                      (long long)blockIdx.x * CPB + args.cell_begin * vper);
 }
 
 // kappa at the Gauss points of the operator, once per operator (and on

@@ -59,6 +59,9 @@ struct FxAcc {
     mid += (long long)x.l * c.h;
   }
   GBFEM_HD long long value() const { return hh + (mid >> 32); }
+  // the sum times 2^K, with K more of its digits
+  template <int K>
+  GBFEM_HD long long value_up() const { return (long long)(uint64_t(hh) << K) + (mid >> (32 - K)); }
 };
 
 GBFEM_HD uint64_t fx_bits(double v) {

@@ -26,6 +26,9 @@ int dg_const_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int
 bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out);
 int dg_fixed_launch(const DgArgsT<double>&, const DgConstTablesT<double>&, const FxTables&, int n, int z0, int z1,
                     cudaStream_t);
+bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out);
+int qx_kappa(gbfem_operator_s* op);
+int dg_quad_fixed_launch(const gbfem_operator_s* op, const DgArgsT<double>& a, cudaStream_t s);
 struct CgScalars;
 int dg_cell_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t, double* partial = nullptr,
                        CgScalars* sc = nullptr);
@@ -76,6 +79,7 @@ int dg_kappa_cache(gbfem_operator_s* op) {
   else
     GBFEM_TRY(dg_kappa_points_f32(static_cast<const float*>(op->dg.kappa), static_cast<float*>(op->kq_cache),
                                   static_cast<float*>(op->kf_cache), op->ncells, op->tab32, op->n, op->q, nullptr));
+  if (op->quad_fixed) GBFEM_TRY(qx_kappa(op));
   GBFEM_CUDA_TRY(cudaDeviceSynchronize());
   return GBFEM_OK;
 }
@@ -261,6 +265,7 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
       GBFEM_TRY(trace_buffer(op, &tb));
       return dg_const_launch_f64(a, ct, op->n, static_cast<double*>(tb), phase, s, static_cast<double*>(ucopy));
     }
+    if (unit_mode == 0 && op->quad_fixed) return dg_quad_fixed_launch(op, a, s);
     return dg_launch_f64(a, op->tab64, op->n, op->q, op->dg.kappa != nullptr, s);
   } else {
     DgArgsT<float> a;
@@ -777,6 +782,7 @@ int gbfem_dg_operator_create(const gbfem_dg_desc* desc, gbfem_operator* out) {
   op->coefficient_space = desc->kappa == nullptr && desc->algorithm != GBFEM_ALGO_QUADRATURE;
   op->two_kernel_f32 = desc->algorithm == GBFEM_ALGO_TRACE_PASS;
   op->fixed = op->precision == GBFEM_F64 && op->coefficient_space && fx_make_tables(op->dg, op->n, &op->fx);
+  op->quad_fixed = op->precision == GBFEM_F64 && desc->kappa != nullptr && qx_make_tables(op->dg, op->n, q, &op->qx);
   const int rc = dg_kappa_cache(op);
   if (rc) {
     gbfem_operator_destroy(op);
@@ -824,6 +830,9 @@ int gbfem_operator_destroy(gbfem_operator op) {
   if (op->owns_kcache) {
     if (op->kq_cache) cudaFree(op->kq_cache);
     if (op->kf_cache) cudaFree(op->kf_cache);
+    if (op->kq_fixed) cudaFree(op->kq_fixed);
+    if (op->kf_fixed) cudaFree(op->kf_fixed);
+    if (op->ke_fixed) cudaFree(op->ke_fixed);
   }
   if (op->jit_lib) cudaLibraryUnload(static_cast<cudaLibrary_t>(op->jit_lib));
   if (op->owns_form_u0 && op->form_u0) cudaFree(op->form_u0);

@@ -6,6 +6,7 @@
 #include "dg_const_kernel.cuh"
 #include "dg_fixed_tables.hpp"
 #include "dg_kernel.cuh"
+#include "dg_quad_tables.hpp"
 
 namespace gbfem {
 
@@ -74,6 +75,13 @@ struct gbfem_operator_s {
   void* jac_points = nullptr;  // Jacobian of a nonlinear DG operator: [cell][q^3] w |K| r'(u0)
   void* kq_cache = nullptr;    // variable kappa at the volume Gauss points [cell][q^3]
   void* kf_cache = nullptr;    // variable kappa at the face Gauss points [cell][6][q^2]
+  // FP64: kappa at the points in fixed point, with a cell's exponent (qx: the
+  // integer-pipe apply at the Gauss points)
+  bool quad_fixed = false;
+  gbfem::QxTables qx{};
+  void* kq_fixed = nullptr;
+  void* kf_fixed = nullptr;
+  void* ke_fixed = nullptr;
   bool owns_kcache = false;    // false in copies (Jacobian) that share the operator's caches
   void* kappa_field = nullptr; // cellwise kappa as a DG field (the mean only), for the Gauss-point paths
   bool owns_kfield = false;
