@@ -3,9 +3,9 @@
 // contractions as dg_apply_kernel (dg_kernel.cuh), which is bound by the FP64
 // pipe (270 multiply-adds per dof at Q3, 0.5 clocks each on an SM).
 //
-// What bounds it: integer issue, about 1400 instructions per dof at Q3 in place of
+// What bounds it: integer issue, about 4000 instructions per dof at Q3 in place of
 // 135 clocks of FP64 pipe.  Measured (GB300), dg_apply_kernel before, this after:
-// 45 x 38 x 33 Q3 QXOLD -> QXNEW us.
+// 45 x 38 x 33 Q3 2152 -> 712 us.
 //
 // Numbers.  All of a cell's values are integers v 2^(s-(E-1022)) of its exponent E
 // (its largest dof's), |integer| <= 2^60; a contraction with a matrix c of row sums
@@ -42,7 +42,8 @@ namespace gbfem {
 __device__ __forceinline__ long long qx_from_double(double v, int E) { return fx_from_double(v, E) >> 1; }
 
 __device__ __forceinline__ uint32_t qx_mag(long long v) {
-  return uint32_t(uint64_t(v < 0 ? -v : v) >> 32) + 1u;  // |v| < qx_mag 2^32
+  const int hi = int(uint64_t(v) >> 32);
+  return uint32_t(hi ^ (hi >> 31)) + 1u;  // |v| <= qx_mag 2^32
 }
 // The traces keep kQxUp more bits than a contraction's result: all coefficients of
 // a face share the unit that the largest needs, and the interpolation to the points
@@ -61,8 +62,10 @@ __device__ __forceinline__ long long qx_shift(long long v, int k) {
 // NC groups of arrays (cell stride ics / ocs) of dims [I0][I1][I2], contracted along
 // AX with M (OUT x IN, entry M[o LDM + i]).  The input is shifted left as far as its
 // largest magnitude room[c] allows (null: not at all); mag[c] takes the output's
-// (null: not kept).  SUB groups per cell, ISUB / OSUB apart, counted by c.
-template <int AX, int I0, int I1, int I2, int OUT, int LDM, int NC, int T, int SUB = 1, int ISUB = 0, int OSUB = 0>
+// (null: not kept).  SUB groups per cell, ISUB / OSUB apart, counted by c.  BOTH: the
+// shift may be to the right.
+template <int AX, int I0, int I1, int I2, int OUT, int LDM, int NC, int T, int SUB = 1, int ISUB = 0, int OSUB = 0,
+          bool BOTH = false>
 __device__ __forceinline__ void qx_contract(const long long* __restrict__ in, int ics, long long* __restrict__ out,
                                             int ocs, const FxCoef* __restrict__ M, const uint32_t* room, uint32_t* mag) {
   constexpr int IN = AX == 0 ? I0 : (AX == 1 ? I1 : I2);
@@ -79,7 +82,7 @@ __device__ __forceinline__ void qx_contract(const long long* __restrict__ in, in
     const int k = room ? qx_room(room[c]) : 0;
     FxLimbs x[IN];
 #pragma unroll
-    for (int i = 0; i < IN; ++i) x[i] = fx_split(qx_shift(src[i * SI], k));
+    for (int i = 0; i < IN; ++i) x[i] = fx_split(BOTH ? qx_shift(src[i * SI], k) : (long long)(uint64_t(src[i * SI]) << (k & 63)));
     uint32_t m = 0;
 #pragma unroll
     for (int o = 0; o < OUT; ++o) {
@@ -118,7 +121,7 @@ __device__ __noinline__ void qx_cell_f64(const DgArgsT<double>& args, const DgTa
 template <int N, int Q>
 struct QxShape {
   static constexpr int CPB = N == 2 ? 32 : (N == 3 ? 16 : (N == 4 ? 8 : 4));
-  static constexpr int T = 128, MINB = 5;
+  static constexpr int T = N == 4 ? 256 : 128, MINB = N == 4 ? 3 : 5;
 };
 
 template <int N, int Q>
@@ -182,9 +185,11 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
     __syncthreads();
     qx_contract<2, Q, Q, N, Q, N, CPB, T>(t2, WS, U, WS, qx.B, magV[1], magV[2]);
     __syncthreads();
-    auto axis = [&](auto dc) {
-      constexpr int D = decltype(dc)::value;
-      constexpr int STR = D == 0 ? Q2 : (D == 1 ? Q : 1);
+    // (one copy of the code for the three axes, and for the three directions below:
+    // unrolled, the kernel does not fit the instruction cache)
+#pragma unroll 1
+    for (int D = 0; D < 3; ++D) {
+      const int STR = D == 0 ? Q2 : (D == 1 ? Q : 1);
       for (int item = tid; item < CPB * Q2; item += T) {
         const int c = item / Q2, ln = item - c * Q2, a = ln / Q, b = ln - a * Q;
         const int base = D == 0 ? ln : (D == 1 ? a * Q2 + b : ln * Q);
@@ -219,10 +224,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
         if (D == 2) atomicMax(magV[3] + c, m);
       }
       __syncthreads();
-    };
-    axis(std::integral_constant<int, 0>());
-    axis(std::integral_constant<int, 1>());
-    axis(std::integral_constant<int, 2>());
+    }
     qx_contract<2, Q, Q, Q, N, Q, CPB, T>(V, WS, t2, WS, qx.BT, magV[3], magV[4]);
     __syncthreads();
     qx_contract<1, Q, Q, N, N, Q, CPB, T>(t2, WS, t1, WS, qx.BT, magV[4], magV[5]);
@@ -252,9 +254,9 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
     __syncthreads();
   }
   // ---- faces, one direction at a time ----------------------------------------------
-  auto faces = [&](auto dc) {
-    constexpr int D = decltype(dc)::value;
-    constexpr int STR = D == 0 ? N2 : (D == 1 ? N : 1);
+#pragma unroll 1
+  for (int D = 0; D < 3; ++D) {
+    const int STR = D == 0 ? N2 : (D == 1 ? N : 1);
     long long* FC = work;              // [2 sides][J, D-, D+][N][N]
     long long* FT = FC + 6 * N2;       // [2][3][Q][N]
     long long* FQ = FT + 6 * Q * N;    // [2][3][Q][Q]
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
     }
     __syncthreads();
     // to the points
-    qx_contract<1, 3, N, N, Q, N, 2 * CPB, T, 2, 3 * N2, 3 * Q * N>(FC, WS, FT, WS, qx.B, magF[0], magF[1]);
+    qx_contract<1, 3, N, N, Q, N, 2 * CPB, T, 2, 3 * N2, 3 * Q * N, true>(FC, WS, FT, WS, qx.B, magF[0], magF[1]);
     __syncthreads();
     qx_contract<2, 3, Q, N, Q, N, 2 * CPB, T, 2, 3 * Q * N, 3 * Q2>(FT, WS, FQ, WS, qx.B, magF[1], magF[2]);
     __syncthreads();
@@ -447,10 +449,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
       }
     }
     __syncthreads();
-  };
-  faces(std::integral_constant<int, 0>());
-  faces(std::integral_constant<int, 1>());
-  faces(std::integral_constant<int, 2>());
+  }
   if (slow) {
     __syncthreads();
     for (int c = 0; c < ncell; ++c) {
