@@ -9,19 +9,6 @@
 
 namespace gbfem {
 
-static FxCoef qx_coef(long double c, int lS) {
-  const long long v = llroundl(ldexpl(c, 62 - lS));
-  const FxLimbs s = fx_split(v);
-  return FxCoef{s.h, s.l};
-}
-// log2 of the smallest power of two >= big, and >= sum / ratio
-static int qx_scale(long double big, long double sum, long double ratio) {
-  int e = 0;
-  const long double need = fmaxl(big, sum / ratio);
-  if (need > 0.0L) frexpl(need, &e);
-  return e;
-}
-
 // false: the form or its coefficients are not for the fixed-point kernel
 bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out) {
   *out = QxTables{};

@@ -1,6 +1,8 @@
 // Coefficient tables of the integer-pipe FP64 apply at the Gauss points
 // (dg_quad_fixed.cuh).
 #pragma once
+#include <cmath>
+
 #include "dg_kernel.cuh"
 #include "fixed_point.cuh"
 
@@ -25,5 +27,18 @@ struct QxArgs {
   const long long *kq, *kf;    // kappa 2^(62-(ke-1022)) at the points
   const unsigned short* ke;    // [cell] kappa's exponent, kQxSlow: not representable
 };
+
+inline FxCoef qx_coef(long double c, int lS) {
+  const long long v = llroundl(ldexpl(c, 62 - lS));
+  const FxLimbs s = fx_split(v);
+  return FxCoef{s.h, s.l};
+}
+// log2 of the smallest power of two >= big, and >= sum / ratio
+inline int qx_scale(long double big, long double sum, long double ratio) {
+  int e = 0;
+  const long double need = fmaxl(big, sum / ratio);
+  if (need > 0.0L) frexpl(need, &e);
+  return e;
+}
 
 }  // namespace gbfem

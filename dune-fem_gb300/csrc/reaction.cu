@@ -14,7 +14,9 @@
 
 #include "gbfem_internal.cuh"
 #include "operator_impl.hpp"
+#include "reaction_fixed.cuh"
 #include "reaction_kernel.cuh"
+#include "tables.hpp"
 
 namespace gbfem {
 
@@ -41,6 +43,45 @@ static void fill_react_tabs(const gbfem_operator_s* op, ReactTabsT<T>* t) {
   t->ce = T(op->react[2]);
 }
 
+// the tables of every (n, q), made once per process
+static const RxTables& rx_tables(int n, int q) {
+  struct All {
+    RxTables t[kDgMaxN + 1][2];  // q = n, n + 1
+    All() {
+      for (int n = 2; n <= kDgMaxN; ++n)
+        for (int k = 0; k < 2; ++k) {
+          RxTables& r = t[n][k];
+          const int q = n + k;
+          const Tables1D s = make_tables(n, q);
+          long double big = 0.0L, row = 0.0L, col = 0.0L;
+          for (int a = 0; a < q; ++a) {
+            long double sum = 0.0L;
+            for (int i = 0; i < n; ++i) {
+              sum += fabsl(s.B[a][i]);
+              big = fmaxl(big, fabsl(s.B[a][i]));
+            }
+            row = fmaxl(row, sum);
+          }
+          for (int i = 0; i < n; ++i) {
+            long double sum = 0.0L;
+            for (int a = 0; a < q; ++a) sum += fabsl(s.B[a][i]);
+            col = fmaxl(col, sum);
+          }
+          r.lB = qx_scale(big, row, 2.5L);
+          r.lBT = qx_scale(big, col, 2.5L);
+          for (int a = 0; a < q; ++a)
+            for (int i = 0; i < n; ++i) {
+              r.B[a * n + i] = qx_coef(s.B[a][i], r.lB);
+              r.BT[i * q + a] = qx_coef(s.B[a][i], r.lBT);
+            }
+          r.exp = fx_make_exp_tables();
+        }
+    }
+  };
+  static const All all;
+  return all.t[n][q - n];
+}
+
 template <typename T, int N, int Q>
 static int reaction_launch_nq(const gbfem_operator_s* op, int mode, const void* u, void* w, void* pts,
                               long long cell_begin, long long count, int blocks_mode, cudaStream_t s) {
@@ -50,6 +91,16 @@ static int reaction_launch_nq(const gbfem_operator_s* op, int mode, const void* 
     if (count > 2147483647LL) return set_error(GBFEM_ERR_INVALID, "reaction blocks: grid too large");
     dg_reaction_blocks_kernel<T, N, Q><<<unsigned(count), 256, 0, s>>>(
         static_cast<const T*>(pts), static_cast<T*>(w), cell_begin, count, blocks_mode == 2, tb);
+  } else if constexpr (sizeof(T) == 8) {
+    using S = RxShape<N, Q>;
+    const long long grid = (count + S::CPB - 1) / S::CPB;
+    if (grid > 2147483647LL) return set_error(GBFEM_ERR_INVALID, "reaction: grid too large");
+    auto kern = mode == 0 ? dg_reaction_fixed_kernel<N, Q, 0>
+                          : (mode == 1 ? dg_reaction_fixed_kernel<N, Q, 1> : dg_reaction_fixed_kernel<N, Q, 2>);
+    GBFEM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(S::BYTES)));
+    kern<<<unsigned(grid), S::T, S::BYTES, s>>>(static_cast<const double*>(u), static_cast<double*>(w),
+                                                static_cast<double*>(pts), cell_begin, count, tb,
+                                                rx_tables(op->n, op->q));
   } else {
     constexpr int CPB = 4;
     const long long grid = (count + CPB - 1) / CPB;
@@ -109,6 +160,13 @@ int reaction_launch(const gbfem_operator_s* op, int mode, const void* u, void* w
 }  // namespace gbfem
 
 using namespace gbfem;
+
+extern "C" int gbfem_selftest_exp(int64_t n, const double* x, double* y) {
+  if (!x || !y) return set_error(GBFEM_ERR_INVALID, "gbfem_selftest_exp: null argument");
+  const FxExpTables t = fx_make_exp_tables();
+  for (int64_t i = 0; i < n; ++i) y[i] = fx_exp(x[i], t, t.pow);
+  return GBFEM_OK;
+}
 
 extern "C" {
 

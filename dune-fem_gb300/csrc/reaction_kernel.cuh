@@ -49,18 +49,17 @@ struct BuiltinReaction {
 
 // R: the pointwise function (value and derivative in u), given the point's
 // physical coordinates when R::kCoordinates.
+// The CPB cells from c0 on, below cend.
 template <typename T, int N, int Q, int CPB, class R>
-__device__ __forceinline__ void dg_reaction_body(int mode, const T* __restrict__ u, T* __restrict__ w,
-                                                 T* __restrict__ pts, long long cell_begin, long long count,
-                                                 const ReactTabsT<T>& tb) {
+__device__ __forceinline__ void dg_reaction_cells(int mode, const T* __restrict__ u, T* __restrict__ w,
+                                                  T* __restrict__ pts, long long c0, long long cend,
+                                                  const ReactTabsT<T>& tb) {
   constexpr int N3 = N * N * N, Q3 = Q * Q * Q;
   __shared__ T sX[CPB * N3];      // coefficients [i][j][k]
   __shared__ T sY1[CPB * Q * N * N];  // [a][j][k]
   __shared__ T sY2[CPB * Q * Q * N];  // [a][b][k]
   __shared__ T sP[CPB * Q3];      // [a][b][c]
   const int tid = threadIdx.x;
-  const long long c0 = cell_begin + (long long)blockIdx.x * CPB;
-  const long long cend = cell_begin + count;
   if (c0 >= cend) return;
   const int ncell = int(cend - c0 < CPB ? cend - c0 : CPB);
   for (int e = tid; e < CPB * N3; e += blockDim.x) sX[e] = e < ncell * N3 ? __ldg(u + c0 * N3 + e) : T(0);
@@ -141,6 +140,14 @@ __device__ __forceinline__ void dg_reaction_body(int mode, const T* __restrict__
     for (int a = 0; a < Q; ++a) s = fma(tb.B[a * N + i], sY1[c * Q * N * N + a * N * N + jk], s);
     w[c0 * N3 + e] += s;
   }
+}
+
+template <typename T, int N, int Q, int CPB, class R>
+__device__ __forceinline__ void dg_reaction_body(int mode, const T* __restrict__ u, T* __restrict__ w,
+                                                 T* __restrict__ pts, long long cell_begin, long long count,
+                                                 const ReactTabsT<T>& tb) {
+  dg_reaction_cells<T, N, Q, CPB, R>(mode, u, w, pts, cell_begin + (long long)blockIdx.x * CPB, cell_begin + count,
+                                     tb);
 }
 
 // 128 threads per CTA, CPB cells per CTA

@@ -510,6 +510,9 @@ int gbfem_cnn_status(gbfem_cnn cnn, int* status);
  * (including values near the binary32 range limits and rounding ties);
  * mismatches is 0 when they agree everywhere. */
 int gbfem_selftest_conversions(uint64_t n, uint64_t seed, uint64_t* mismatches);
+/* y[i] = exp(x[i]) by the integer-arithmetic exp of the FP64 reaction kernels,
+ * evaluated on the host (the device runs the same code). */
+int gbfem_selftest_exp(int64_t n, const double* x, double* y);
 int gbfem_cnn_set_output_scale(gbfem_cnn cnn, double scale);
 int gbfem_cnn_get_output_scale(gbfem_cnn cnn, double* scale);
 /* z = S rms(r) NN(r/rms(r)) (accumulate = 1: z += ...). */
