@@ -1,16 +1,15 @@
-// One-kernel FP32 apply of the constant-coefficient closed form (the same
+// One-kernel FP32 apply of the constant-coefficient closed form, p = 1 (the same
 // operator as dg_trace_kernel + dg_const_kernel; the algebra is described in
 // dg_const_kernel.cuh), without the trace buffer in HBM.
 //
 // Layout of the work: a CTA of 128 threads owns a brick of 8 x 4 x 4 cells,
 // one cell per thread, and keeps the cell's n^3 dofs and n^3 results in
-// registers (n <= 4: 128 registers at Q3).  A face's numerical flux is
+// registers.  A face's numerical flux is
 // computed once and exchanged through shared memory, which holds one slot per
 // face of the brick ((8+1) 4 4 + 8 (4+1) 4 + 8 4 (4+1) = 464 slots of 2 n^2
-// values) plus one per face on the brick's lower boundary (80; 69.6 KB at Q3,
-// three CTAs per SM).  Slots are 128-byte rows whose 16-byte chunks are
-// XOR-swizzled by the slot index, so lanes at consecutive slots read
-// distinct banks without padding.
+// values) plus one per face on the brick's lower boundary (80; 17.4 KB at Q1).
+// Slots are rows of 16-byte chunks, XOR-swizzled by the slot index, so lanes at
+// consecutive slots read distinct banks without padding.
 //  0. every thread loads its cell's dofs (float4 loads where the cell's block
 //     is 16-byte aligned).  Halo items, spread over the threads, load the
 //     brick's face neighbours outside it (2 (8*4 + 8*4 + 4*4) cells per 128,

@@ -30,10 +30,9 @@ bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out);
 int qx_kappa(gbfem_operator_s* op);
 int dg_quad_fixed_launch(const gbfem_operator_s* op, const DgArgsT<double>& a, cudaStream_t s);
 struct CgScalars;
-int dg_cell_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t, double* partial = nullptr,
-                       CgScalars* sc = nullptr);
-long long dg_cell_blocks(const int* nc);
-bool dg_cell_supported(int n);
+int dg_one_kernel_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, cudaStream_t,
+                             double* partial = nullptr, CgScalars* sc = nullptr);
+long long dg_one_kernel_blocks(int n, const int* nc);
 int dg_kappa_points_f64(const double*, double*, double*, long long, const DgTablesT<double>&, int, int, cudaStream_t);
 int dg_kappa_points_f32(const float*, float*, float*, long long, const DgTablesT<float>&, int, int, cudaStream_t);
 
@@ -279,12 +278,11 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
     if (unit_mode == 0 && op->coefficient_space) {
       DgConstTablesT<float> ct = op->ctab32;
       fill_line_operators(op, &ct);
-      // the whole grid in one kernel (no trace buffer) where the cell's dofs
-      // and results fit in registers; slabs of the host pipeline and p = 4
-      // take the two-kernel form
+      // the whole grid in one kernel (no trace buffer); slabs of the host
+      // pipeline take the two-kernel form
       if (phase == 3 && cell_begin == 0 && (cell_count == 0 || cell_count == op->ncells) && !ucopy &&
-          dg_cell_supported(op->n) && !op->two_kernel_f32)
-        return dg_cell_launch_f32(a, ct, op->n, s);
+          !op->two_kernel_f32)
+        return dg_one_kernel_launch_f32(a, ct, op->n, s);
       void* tb = nullptr;
       GBFEM_TRY(trace_buffer(op, &tb));
       return dg_const_launch_f32(a, ct, op->n, static_cast<float*>(tb), phase, s, static_cast<float*>(ucopy));
@@ -293,12 +291,12 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
   }
 }
 
-// The device-resident CG's operator: the one-kernel FP32 closed form, which has a
-// cell's dofs and results in one thread's registers, with <q, h> in its end.
+// The device-resident CG's operator: the one-kernel FP32 closed form, with
+// <q, h> in its end.
 long long cg_apply_dot_parts(const gbfem_operator_s* op) {
   const bool cell = op->kind == OpKind::DG && op->precision == GBFEM_F32 && op->coefficient_space && !op->form &&
-                    !op->nonlinear && !op->jac_points && dg_cell_supported(op->n) && !op->two_kernel_f32;
-  return cell ? dg_cell_blocks(op->dg.grid.cells) : 0;
+                    !op->nonlinear && !op->jac_points && !op->two_kernel_f32;
+  return cell ? dg_one_kernel_blocks(op->n, op->dg.grid.cells) : 0;
 }
 int cg_apply_dot(const gbfem_operator_s* op, const void* q, void* h, double* partial, CgScalars* sc, cudaStream_t s) {
   DgArgsT<float> a;
@@ -307,7 +305,7 @@ int cg_apply_dot(const gbfem_operator_s* op, const void* q, void* h, double* par
   a.w = static_cast<float*>(h);
   DgConstTablesT<float> ct = op->ctab32;
   fill_line_operators(op, &ct);
-  return dg_cell_launch_f32(a, ct, op->n, s, partial, sc);
+  return dg_one_kernel_launch_f32(a, ct, op->n, s, partial, sc);
 }
 
 // ---- continuous Q1 (2-D) ---------------------------------------------------

@@ -92,8 +92,8 @@ typedef struct {
  * mass), which equals the quadrature result up to rounding; otherwise the
  * sum-factorised quadrature kernel.  The closed form is one kernel in FP64
  * with a constant kappa (in 64-bit fixed point on the integer pipes) and in
- * FP32 with p <= 3 over the whole grid; otherwise a trace pass into an
- * operator-owned buffer followed by the apply.
+ * FP32 over the whole grid; otherwise a trace pass into an operator-owned
+ * buffer followed by the apply.
  * GBFEM_ALGO_QUADRATURE always evaluates at the q^3 volume / q^2 face Gauss
  * points.  GBFEM_ALGO_TRACE_PASS is the FP32 closed form always in its
  * trace-pass form (in FP64 it is GBFEM_ALGO_AUTO). */
