@@ -86,17 +86,32 @@ __global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, 
   }
 }
 
+// The normalisation of a forward pass, in device memory.  The factors are computed
+// once, by the kernel that finishes the sum: an FP64 division and square root in every
+// thread of the elementwise kernels made those 20 and 23 us at 32^3 Q3, against 6 and 7.
+struct CnnNorm {
+  double rr;      // sum of the squares
+  float inv, sc;  // 1 / rms(r); output scale * rms(r)
+  unsigned done;  // CTAs that have handed in their partial sum
+};
+__device__ __forceinline__ void cnn_set_norm(CnnNorm* norm, double rr, long long n, float S) {
+  const double ms = rr / double(n);
+  norm->rr = rr;
+  norm->inv = ms > 0.0 ? float(1.0 / sqrt(ms)) : 0.f;
+  norm->sc = float(double(S) * sqrt(ms));
+}
+
 // x0[p][c]: c < nloc: r[p*nloc+c] / rms(r); c == nloc: log kappa_mean[p]; else 0.
 // Channel pairs; each thread handles kEwUnroll of them per iteration and
 // issues all their loads first.  The dof values are rounded to FP32 in
 // integer arithmetic (convert.cuh), the product is FP32.
 constexpr int kEwUnroll = 4;
 template <typename T>
-__global__ void assemble_input_kernel(const T* __restrict__ r, const float* __restrict__ logk,
-                                      const double* __restrict__ rr, long long n, int nloc, int cin,
-                                      long long P, int coarse, bf16* __restrict__ x0) {
-  const double ms = rr[0] / double(n);
-  const float inv = ms > 0.0 ? float(1.0 / sqrt(ms)) : 0.f;
+__global__ void assemble_input_kernel(const T* __restrict__ r, const float* __restrict__ logk, const CnnNorm* norm,
+                                      int nloc, int cin, long long P, int coarse, bf16* x0) {
+  cnn_release();
+  cnn_wait(norm, x0);
+  const float inv = norm->inv;
   const unsigned half = unsigned(cin) / 2u, total = unsigned(P) * half, nl = unsigned(nloc);
   __nv_bfloat162* x2 = reinterpret_cast<__nv_bfloat162*>(x0);
   const unsigned stride = gridDim.x * blockDim.x;
@@ -134,54 +149,82 @@ __global__ void assemble_input_kernel(const T* __restrict__ r, const float* __re
   }
 }
 
-// Partial sums of r_i^2 in FP32 (values rounded to FP32 in integer
-// arithmetic): one per block, fixed order; the normalisation rms(r) needs no
-// more precision, and an FP64 product per dof would bind on the FP64 pipe.
+// sum r_i^2: partial sums in FP32 (values rounded to FP32 in integer
+// arithmetic); the normalisation rms(r) needs no more precision, and an FP64
+// product per dof would bind on the FP64 pipe.  nparts parts, kSumParts of them
+// by one block; the last block adds them in a fixed order and writes the
+// factors (parts, kSumParts a block instead of one: fewer blocks meet at the
+// counter).
+constexpr int kSumParts = 4;
 template <typename T>
-__global__ void sumsq_partial_kernel(const T* __restrict__ r, unsigned n, double* __restrict__ part) {
-  __shared__ float red[256];
-  float acc[kEwUnroll] = {0.f, 0.f, 0.f, 0.f};
-  const unsigned stride = gridDim.x * blockDim.x;
-  for (unsigned e0 = blockIdx.x * blockDim.x * kEwUnroll + threadIdx.x; e0 < n; e0 += stride * kEwUnroll) {
-    T a[kEwUnroll];
+__global__ void __launch_bounds__(256) sumsq_kernel(const T* __restrict__ r, unsigned n, unsigned nparts,
+                                                    double* __restrict__ part, CnnNorm* norm, float S) {
+  cnn_release();
+  __shared__ float red[kSumParts][256];
+  __shared__ double sum[256];
+  __shared__ unsigned last;
+  float acc[kSumParts][kEwUnroll];
 #pragma unroll
-    for (int u = 0; u < kEwUnroll; ++u) {
-      const unsigned e = e0 + u * blockDim.x;
-      a[u] = e < n ? r[e] : T(0);
-    }
+  for (int v = 0; v < kSumParts; ++v)
 #pragma unroll
-    for (int u = 0; u < kEwUnroll; ++u) {
-      const float v = to_f32(a[u]);
-      acc[u] = fmaf(v, v, acc[u]);
-    }
+    for (int u = 0; u < kEwUnroll; ++u) acc[v][u] = 0.f;
+  const unsigned per = 256 * kEwUnroll, first = blockIdx.x * kSumParts * per + threadIdx.x;
+  for (unsigned base = 0; base < n; base += nparts * per) {
+    T a[kSumParts][kEwUnroll];
+#pragma unroll
+    for (int v = 0; v < kSumParts; ++v)
+#pragma unroll
+      for (int u = 0; u < kEwUnroll; ++u) {
+        const unsigned e = base + first + v * per + u * 256;
+        a[v][u] = blockIdx.x * kSumParts + v < nparts && e < n ? r[e] : T(0);
+      }
+#pragma unroll
+    for (int v = 0; v < kSumParts; ++v)
+#pragma unroll
+      for (int u = 0; u < kEwUnroll; ++u) {
+        const float t = to_f32(a[v][u]);
+        acc[v][u] = fmaf(t, t, acc[v][u]);
+      }
   }
-  red[threadIdx.x] = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+#pragma unroll
+  for (int v = 0; v < kSumParts; ++v) red[v][threadIdx.x] = (acc[v][0] + acc[v][1]) + (acc[v][2] + acc[v][3]);
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
-    if (int(threadIdx.x) < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (int(threadIdx.x) < o)
+#pragma unroll
+      for (int v = 0; v < kSumParts; ++v) red[v][threadIdx.x] += red[v][threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) part[blockIdx.x] = double(red[0]);
-}
-
-// out[0] = sum of the partials in block order
-__global__ void sum_partials_kernel(const double* __restrict__ part, int np, double* __restrict__ out) {
-  __shared__ double red[256];
+  if (threadIdx.x < kSumParts && blockIdx.x * kSumParts + threadIdx.x < nparts) {
+    __stcg(part + blockIdx.x * kSumParts + threadIdx.x, double(red[threadIdx.x][0]));
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(&norm->done, 1u) == gridDim.x - 1 ? 1u : 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
   double s = 0.0;
-  for (int i = threadIdx.x; i < np; i += 256) s += part[i];
-  red[threadIdx.x] = s;
+#pragma unroll 8
+  for (unsigned i = threadIdx.x; i < nparts; i += 256) s += __ldcg(part + i);
+  sum[threadIdx.x] = s;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
-    if (int(threadIdx.x) < o) red[threadIdx.x] += red[threadIdx.x + o];
+    if (int(threadIdx.x) < o) sum[threadIdx.x] += sum[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = red[0];
+  if (threadIdx.x == 0) {
+    cnn_set_norm(norm, sum[0], n, S);
+    norm->done = 0;
+  }
 }
 
-// out[0] = sum_p r[p*nloc]^2: the coarse mode's normalisation (the cell
+// sum_p r[p*nloc]^2: the coarse mode's normalisation (the cell
 // means of r only), one CTA of 256 threads, fixed summation order
 template <typename T>
-__global__ void coarse_sumsq_kernel(const T* __restrict__ r, int nloc, long long P, double* __restrict__ out) {
+__global__ void coarse_sumsq_kernel(const T* __restrict__ r, int nloc, long long P, CnnNorm* norm, float S) {
   __shared__ double part[256];
   double s = 0.0;
   for (long long p = threadIdx.x; p < P; p += 256) {
@@ -194,16 +237,18 @@ __global__ void coarse_sumsq_kernel(const T* __restrict__ r, int nloc, long long
     if (threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = part[0];
+  if (threadIdx.x == 0) cnn_set_norm(norm, part[0], P, S);
 }
 
 // z[p*nloc+l] (+)= S * rms(r) * y[p][l]: the scale and the product in FP32,
 // widened to T in integer arithmetic (an FP64 add only when accumulating);
 // kEwUnroll values per thread and iteration, loads first
 template <typename T>
-__global__ void emit_output_kernel(const float* __restrict__ y, const double* __restrict__ rr, long long n, int nloc,
-                                   int cout, long long P, float S, int accumulate, int coarse, T* __restrict__ z) {
-  const float sc = float(double(S) * sqrt(rr[0] / double(n)));
+__global__ void emit_output_kernel(const float* y, const CnnNorm* norm, int nloc, int cout, long long P, int accumulate,
+                                   int coarse, T* z) {
+  cnn_wait(y, norm);
+  cnn_wait(z);
+  const float sc = norm->sc;
   const unsigned nl = unsigned(nloc), total = unsigned(P) * nl, co = unsigned(cout);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned e0 = blockIdx.x * blockDim.x * kEwUnroll + threadIdx.x; e0 < total; e0 += stride * kEwUnroll) {
@@ -298,7 +343,7 @@ struct gbfem_cnn_s {
   float* wpart = nullptr;    // weight-gradient partials
   long long wpart_elems = 0;
   float* logk = nullptr;
-  double* d_rr = nullptr;    // r.r
+  CnnNorm* d_norm = nullptr;
   double* d_loss = nullptr;
   double* d_partial = nullptr;
   double* h_loss = nullptr;
@@ -320,6 +365,23 @@ static int cnn_alloc(gbfem_cnn_s* c, void** p, size_t bytes) {
   return GBFEM_OK;
 }
 
+// a kernel of the forward pass's chain (cnn_wait)
+template <typename... K, typename... A>
+static int launch_chained(void (*kernel)(K...), long long grid, int block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(unsigned(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  GBFEM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, K(args)...));
+  return GBFEM_OK;
+}
+
 template <int CIN, int COUT, int TAPS, bool RELU, typename TOUT>
 static int launch_conv(const bf16* in, const bf16* w, TOUT* out, int N, cudaStream_t s) {
   const size_t sm = size_t(TAPS) * COUT * CIN * sizeof(bf16);
@@ -327,7 +389,7 @@ static int launch_conv(const bf16* in, const bf16* w, TOUT* out, int N, cudaStre
   GBFEM_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   const long long P = (long long)N * N * N;
   const unsigned blocks = unsigned((P + 63) / 64);
-  k<<<blocks, 128, sm, s>>>(in, w, out, N);
+  GBFEM_TRY(launch_chained(k, blocks, 128, sm, s, in, w, out, N));
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
@@ -374,14 +436,22 @@ static int conv_map(gbfem_cnn_s* c, const bf16* ptr, int N) {
 
 // The 3x3x3 32 -> 32 convolution (forward: RELU; backward-data: the
 // flipped weights, no RELU) on the engine the network is set to: TMA +
-// tcgen05 where the level allows it (N a power of two >= 8), else mma.sync.
+// tcgen05 where the level allows it (N a power of two >= 8), else mma.sync,
+// with 16 positions per CTA while that is at most one CTA per SM (measured on the
+// forward pass, 64 positions per CTA throughout against this: levels 16, 8, 4, 2
+// 108 -> 65 us; 40, 20, 10, 5 315 -> 256; 48, 24, 12, 6 396 -> 345, but 396 again with
+// the 24^3 grid's 864 CTAs of 16 too, 80, 40, 20, 10 1260 and 1528).
 template <bool RELU>
 static int launch_conv27(gbfem_cnn_s* c, const bf16* in, const bf16* w, bf16* out, int N, cudaStream_t s) {
   const CUtensorMap* map = nullptr;
   if (c->conv_engine == GBFEM_CNN_CONV_TENSOR_CORE)
     for (const auto& m : c->conv_maps)
       if (m.ptr == in && m.N == N) map = &m.map;
-  if (!map) return launch_conv<C, C, 27, RELU, bf16>(in, w, out, N, s);
+  const long long P = (long long)N * N * N;
+  if (!map) {
+    if (P > 16 * kSmallConvCtas) return launch_conv<C, C, 27, RELU, bf16>(in, w, out, N, s);
+    return launch_chained(conv27_small_kernel<RELU>, (P + 15) / 16, 128, 0, s, in, w, out, N);
+  }
   static_assert(C == kCtN, "the tensor-core convolution is 32 -> 32 channels");
   static int sms = 0;
   if (sms == 0) {
@@ -392,13 +462,10 @@ static int launch_conv27(gbfem_cnn_s* c, const bf16* in, const bf16* w, bf16* ou
     else
       sms = 152;
   }
-  const long long P = (long long)N * N * N;
   const long long ntiles = P / kCtM;
   const long long grid = ntiles < sms ? ntiles : sms;
   GBFEM_CUDA_TRY(cudaFuncSetAttribute(conv_tma_kernel<RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kCtSmem)));
-  conv_tma_kernel<RELU><<<unsigned(grid), kCtThreads, kCtSmem, s>>>(*map, w, out, N, c->status);
-  GBFEM_CUDA_TRY(cudaGetLastError());
-  return GBFEM_OK;
+  return launch_chained(conv_tma_kernel<RELU>, grid, kCtThreads, kCtSmem, s, *map, w, out, N, c->status);
 }
 
 // positions per weight-gradient chunk for a grid of P positions
@@ -446,17 +513,17 @@ static int cnn_forward(gbfem_cnn_s* c, cudaStream_t s) {
   const int* N = c->N;
   GBFEM_TRY(conv_in_fwd(c, s));
   GBFEM_TRY((launch_conv27<true>(c, c->a0, c->L[1].wb, c->s1, N[0], s)));
-  pool_fwd_kernel<<<grid1(c->P[1] * C), 256, 0, s>>>(c->s1, c->p1, N[0], C);
+  GBFEM_TRY(launch_chained(pool_fwd_kernel, grid1(c->P[1] * C), 256, 0, s, c->s1, c->p1, N[0], C));
   GBFEM_TRY((launch_conv27<true>(c, c->p1, c->L[2].wb, c->s2, N[1], s)));
-  pool_fwd_kernel<<<grid1(c->P[2] * C), 256, 0, s>>>(c->s2, c->p2, N[1], C);
+  GBFEM_TRY(launch_chained(pool_fwd_kernel, grid1(c->P[2] * C), 256, 0, s, c->s2, c->p2, N[1], C));
   GBFEM_TRY((launch_conv27<true>(c, c->p2, c->L[3].wb, c->s3, N[2], s)));
-  pool_fwd_kernel<<<grid1(c->P[3] * C), 256, 0, s>>>(c->s3, c->p3, N[2], C);
+  GBFEM_TRY(launch_chained(pool_fwd_kernel, grid1(c->P[3] * C), 256, 0, s, c->s3, c->p3, N[2], C));
   GBFEM_TRY((launch_conv27<true>(c, c->p3, c->L[4].wb, c->b4, N[3], s)));
-  up_add_kernel<<<grid1(c->P[2] * C), 256, 0, s>>>(c->b4, c->s3, c->u3, N[2], C);
+  GBFEM_TRY(launch_chained(up_add_kernel, grid1(c->P[2] * C), 256, 0, s, c->b4, c->s3, c->u3, N[2], C));
   GBFEM_TRY((launch_conv27<true>(c, c->u3, c->L[5].wb, c->d3, N[2], s)));
-  up_add_kernel<<<grid1(c->P[1] * C), 256, 0, s>>>(c->d3, c->s2, c->u2, N[1], C);
+  GBFEM_TRY(launch_chained(up_add_kernel, grid1(c->P[1] * C), 256, 0, s, c->d3, c->s2, c->u2, N[1], C));
   GBFEM_TRY((launch_conv27<true>(c, c->u2, c->L[6].wb, c->d2, N[1], s)));
-  up_add_kernel<<<grid1(c->P[0] * C), 256, 0, s>>>(c->d2, c->s1, c->u1, N[0], C);
+  GBFEM_TRY(launch_chained(up_add_kernel, grid1(c->P[0] * C), 256, 0, s, c->d2, c->s1, c->u1, N[0], C));
   GBFEM_TRY((launch_conv27<true>(c, c->u1, c->L[7].wb, c->d1, N[0], s)));
   GBFEM_TRY(conv_out_fwd(c, s));
   GBFEM_CUDA_TRY(cudaGetLastError());
@@ -548,16 +615,14 @@ static long long cnn_nnorm(const gbfem_cnn_s* c) { return c->coarse ? c->P[0] : 
 template <typename T>
 static int cnn_input(gbfem_cnn_s* c, const void* r, cudaStream_t s) {
   if (c->coarse)
-    coarse_sumsq_kernel<T><<<1, 256, 0, s>>>(static_cast<const T*>(r), c->nloc, c->P[0], c->d_rr);
-  else
-  {
-    const int np = grid1(c->ndofs / kEwUnroll);
-    sumsq_partial_kernel<T><<<np, 256, 0, s>>>(static_cast<const T*>(r), unsigned(c->ndofs), c->d_partial);
-    sum_partials_kernel<<<1, 256, 0, s>>>(c->d_partial, np, c->d_rr);
+    coarse_sumsq_kernel<T><<<1, 256, 0, s>>>(static_cast<const T*>(r), c->nloc, c->P[0], c->d_norm, c->S);
+  else {
+    const unsigned np = grid1(c->ndofs / kEwUnroll);
+    sumsq_kernel<T><<<(np + kSumParts - 1) / kSumParts, 256, 0, s>>>(static_cast<const T*>(r), unsigned(c->ndofs), np,
+                                                                     c->d_partial, c->d_norm, c->S);
   }
-  assemble_input_kernel<T><<<grid1(c->P[0] * c->cin0 / 2 / kEwUnroll), 256, 0, s>>>(static_cast<const T*>(r), c->logk, c->d_rr,
-                                                                    cnn_nnorm(c), c->nloc, c->cin0, c->P[0], c->coarse,
-                                                                    c->x0);
+  GBFEM_TRY(launch_chained(assemble_input_kernel<T>, grid1(c->P[0] * c->cin0 / 2 / kEwUnroll), 256, 0, s,
+                           static_cast<const T*>(r), c->logk, c->d_norm, c->nloc, c->cin0, c->P[0], c->coarse, c->x0));
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
@@ -567,11 +632,11 @@ static int cnn_apply(gbfem_cnn_s* c, int precision, const void* r, void* z, int 
   else GBFEM_TRY(cnn_input<float>(c, r, s));
   GBFEM_TRY(cnn_forward(c, s));
   if (precision == GBFEM_F64)
-    emit_output_kernel<double><<<grid1(c->ndofs / kEwUnroll), 256, 0, s>>>(c->y, c->d_rr, cnn_nnorm(c), c->nloc, c->cout0, c->P[0],
-                                                               c->S, accumulate, c->coarse, static_cast<double*>(z));
+    GBFEM_TRY(launch_chained(emit_output_kernel<double>, grid1(c->ndofs / kEwUnroll), 256, 0, s, c->y, c->d_norm, c->nloc,
+                             c->cout0, c->P[0], accumulate, c->coarse, static_cast<double*>(z)));
   else
-    emit_output_kernel<float><<<grid1(c->ndofs / kEwUnroll), 256, 0, s>>>(c->y, c->d_rr, cnn_nnorm(c), c->nloc, c->cout0, c->P[0],
-                                                              c->S, accumulate, c->coarse, static_cast<float*>(z));
+    GBFEM_TRY(launch_chained(emit_output_kernel<float>, grid1(c->ndofs / kEwUnroll), 256, 0, s, c->y, c->d_norm, c->nloc,
+                             c->cout0, c->P[0], accumulate, c->coarse, static_cast<float*>(z)));
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
@@ -584,11 +649,11 @@ static int cnn_loss_grad(gbfem_cnn_s* c, int precision, const void* r, const voi
   GBFEM_TRY(cnn_forward(c, s));
   const long long ny = c->P[0] * c->cout0;
   if (precision == GBFEM_F64)
-    loss_grad_kernel<double><<<grid1(ny), 256, 0, s>>>(c->y, static_cast<const double*>(target), c->d_rr,
+    loss_grad_kernel<double><<<grid1(ny), 256, 0, s>>>(c->y, static_cast<const double*>(target), &c->d_norm->rr,
                                                        cnn_nnorm(c), c->nloc, c->cout0, c->P[0], c->S, c->coarse,
                                                        c->diff, c->dy);
   else
-    loss_grad_kernel<float><<<grid1(ny), 256, 0, s>>>(c->y, static_cast<const float*>(target), c->d_rr,
+    loss_grad_kernel<float><<<grid1(ny), 256, 0, s>>>(c->y, static_cast<const float*>(target), &c->d_norm->rr,
                                                       cnn_nnorm(c), c->nloc, c->cout0, c->P[0], c->S, c->coarse,
                                                       c->diff, c->dy);
   GBFEM_CUDA_TRY(cudaGetLastError());
@@ -735,11 +800,11 @@ int gbfem_cnn_create(int order, int cells, uint64_t seed, gbfem_cnn* out) {
   c->wpart_elems = wp;
   A((void**)&c->wpart, wp * 4);
   A((void**)&c->logk, c->P[0] * 4);
-  A((void**)&c->d_rr, 64);
+  A((void**)&c->d_norm, sizeof(CnnNorm));
   A((void**)&c->d_loss, 64);
   A((void**)&c->status, 64);
   // partials of the loss reduction (gbfem's dot) and of the input's sum of
-  // squares (one per block of sumsq_partial_kernel, at most stream_grid(ndofs))
+  // squares (at most stream_grid(ndofs))
   A((void**)&c->d_partial, sizeof(double) * (std::max<long long>(dot_num_partials(std::max(c->ndofs, c->P[0] * c->cout0)),
                                                                   stream_grid(c->ndofs)) + 8));
   if (rc == GBFEM_OK) {
@@ -772,6 +837,7 @@ int gbfem_cnn_create(int order, int cells, uint64_t seed, gbfem_cnn* out) {
   }
   if (rc == GBFEM_OK) {
     cudaError_t e = cudaMemset(c->status, 0, sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(c->d_norm, 0, sizeof(CnnNorm));
     if (e != cudaSuccess) rc = set_cuda_error(e, "gbfem_cnn_create");
   }
   // tensor maps of the 3x3x3 convolutions' inputs (forward, backward-data)
@@ -879,10 +945,10 @@ int gbfem_cnn_train_step_grad(gbfem_cnn c, int precision, const void* r, const v
   GBFEM_TRY(cnn_forward(c, s));
   const long long ny = c->P[0] * c->cout0;
   if (precision == GBFEM_F64)
-    grad_from_dofs_kernel<double><<<grid1(ny), 256, 0, s>>>(static_cast<const double*>(grad_z), c->d_rr, cnn_nnorm(c),
+    grad_from_dofs_kernel<double><<<grid1(ny), 256, 0, s>>>(static_cast<const double*>(grad_z), &c->d_norm->rr, cnn_nnorm(c),
                                                             c->nloc, c->cout0, c->P[0], c->S, c->coarse, c->dy);
   else
-    grad_from_dofs_kernel<float><<<grid1(ny), 256, 0, s>>>(static_cast<const float*>(grad_z), c->d_rr, cnn_nnorm(c),
+    grad_from_dofs_kernel<float><<<grid1(ny), 256, 0, s>>>(static_cast<const float*>(grad_z), &c->d_norm->rr, cnn_nnorm(c),
                                                            c->nloc, c->cout0, c->P[0], c->S, c->coarse, c->dy);
   GBFEM_CUDA_TRY(cudaGetLastError());
   GBFEM_TRY(cnn_backward(c, s));
