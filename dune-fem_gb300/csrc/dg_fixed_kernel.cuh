@@ -9,7 +9,7 @@
 // cost 3.75 clocks; two FP64 instructions remain, the conversion of the result
 // and its addition (the FP64 pipe is half busy).  The traces never leave the
 // SM.  Measured (GB300, two-kernel form before, this kernel after): 64^3 Q3
-// 822 -> 319 us, 80^3 Q2 with advection 1050 -> 344 us.
+// 822 -> 295 us, 80^3 Q2 with advection 1050 -> 315 us.
 //
 // A line is the n coefficients of a cell along one axis.  With the line's own
 // coefficients x, its face traces (v, P) and those of its two neighbours on
@@ -56,8 +56,8 @@ namespace gbfem {
 // lines of L layers of the brick (X Y L n^2 threads, in whole warps) and take
 // Z / L of them each, so that a thread's lines differ in z only.  Small CTAs
 // hide each other's barriers and loads better than large ones, whose halo is
-// smaller: 64^3 Q3 takes 319 us with 4 x 4 x 2 cells and 5 CTAs per SM, 354 with
-// 4 x 4 x 4 and 2, 363 with 4 x 2 x 2 and 8.  SMALL: grids of less than one
+// smaller: 64^3 Q3 takes 295 us with 4 x 4 x 2 cells and 5 CTAs per SM, 306 with 4,
+// 326 with 4 x 4 x 1, 382 with 4 x 4 x 4, 317 with 4 x 2 x 2 in one pass.  SMALL: grids of less than one
 // full brick per SM, where the time is that of one CTA (6 x 5 x 7 Q2: 11.3 us a
 // call against 20.4 with full bricks).
 template <int N, bool SMALL>

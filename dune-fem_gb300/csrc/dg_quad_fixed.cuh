@@ -3,9 +3,10 @@
 // contractions as dg_apply_kernel (dg_kernel.cuh), which is bound by the FP64
 // pipe (270 multiply-adds per dof at Q3, 0.5 clocks each on an SM).
 //
-// What bounds it: integer issue, about 4000 instructions per dof at Q3 in place of
-// 135 clocks of FP64 pipe.  Measured (GB300), dg_apply_kernel before, this after:
-// 45 x 38 x 33 Q3 2152 -> 712 us.
+// What bounds it: integer issue and the barriers between the contractions (2.1
+// instructions a clock and SM), about 3600 instructions per dof at Q3 in place of 135
+// clocks of FP64 pipe.  Measured (GB300), dg_apply_kernel before, this after:
+// 45 x 38 x 33 Q3 2152 -> 620 us.
 //
 // Numbers.  All of a cell's values are integers v 2^(s-(E-1022)) of its exponent E
 // (its largest dof's), |integer| <= 2^60; a contraction with a matrix c of row sums
@@ -86,7 +87,7 @@ __device__ __forceinline__ void qx_contract(const long long* __restrict__ in, in
     uint32_t m = 0;
 #pragma unroll
     for (int o = 0; o < OUT; ++o) {
-      FxAcc acc(0, 1ll << 31);
+      FxAcc acc = FxAcc::rounded();
 #pragma unroll
       for (int i = 0; i < IN; ++i) acc.add(x[i], M[o * LDM + i]);
       const long long v = acc.value();
@@ -203,17 +204,17 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
 #pragma unroll
         for (int o = 0; o < Q; ++o) {
           const FxLimbs kl = fx_split(__ldg(kp + o * STR));
-          FxAcc g(0, 1ll << 31);
+          FxAcc g = FxAcc::rounded();
 #pragma unroll
           for (int i = 0; i < Q; ++i) g.add(x[i], qx.D[o * Q + i]);
-          FxAcc fl(0, 1ll << 31);
+          FxAcc fl = FxAcc::rounded();
           fl.add(fx_split(g.value()), FxCoef{kl.h, kl.l});
           f[o] = fx_split(fl.value() * 4);
         }
         uint32_t m = 0;
 #pragma unroll
         for (int o = 0; o < Q; ++o) {
-          FxAcc acc(0, 1ll << 31);
+          FxAcc acc = FxAcc::rounded();
 #pragma unroll
           for (int i = 0; i < Q; ++i) acc.add(f[i], qx.Dt[D][o * Q + i]);
           long long v = acc.value();
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
       const double scale = fx_pow2((sE[c] + 1 - s) << 20);
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        FxAcc acc(0, 1ll << 31);
+        FxAcc acc = FxAcc::rounded();
 #pragma unroll
         for (int a = 0; a < Q; ++a) acc.add(x[a], qx.BT[i * Q + a]);
         sr[c * N3 + i * N2 + jk] = double(acc.value()) * scale;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
       const FxLimbs dm = fx_split(-(long long)(uint64_t(fq[Q2]) << shQ));
       const FxLimbs dp = fx_split(-(long long)(uint64_t(fq[2 * Q2]) << shQ));
       const FxLimbs a = fx_split(km), b = fx_split(kp), m = fx_split((km + kp) >> 1);
-      FxAcc val(0, 1ll << 31), grad(0, 1ll << 31);
+      FxAcc val = FxAcc::rounded(), grad = FxAcc::rounded();
       val.add(J, FxCoef{m.h, m.l});
       val.add(dm, FxCoef{a.h, a.l});
       val.add(dp, FxCoef{b.h, b.l});
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(QxShape<N, Q>::T, QxShape<N, Q>::MINB) dg_quad
       double* rc = sr + c * N3 + base;
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        FxAcc acc(0, 1ll << 31);
+        FxAcc acc = FxAcc::rounded();
         acc.add((i & 1) ? vd : vs, qx.fv[D][i]);
         if (i) acc.add((i & 1) ? gd : gs, qx.fg[D][i]);
         // / 2^64 with CB = 62: 2^2, and the row's S

@@ -49,14 +49,45 @@ GBFEM_HD FxLimbs fx_split(long long v) {
   return r;
 }
 
-// running sums of a dot product; `start` joins the result
+// acc + a b, and a b.  Written out: left to itself the compiler widens one factor
+// first and multiplies 64 by 32 bits in three instructions (64^3 Q3 closed form 319
+// -> 295 us with these two, kappa at the Gauss points 712 -> 620).
+GBFEM_HD long long fx_mad(int a, int b, long long acc) {
+#if defined(__CUDA_ARCH__)
+  asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
+  return acc;
+#else
+  return acc + (long long)a * b;
+#endif
+}
+GBFEM_HD long long fx_mul(int a, int b) {
+#if defined(__CUDA_ARCH__)
+  long long r;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+#else
+  return (long long)a * b;
+#endif
+}
+
+// running sums of a dot product; `start` joins the result.  (no_hh, no_mid: nothing
+// in that sum yet; known at compile time in unrolled code, they save the zeros.)
 struct FxAcc {
   long long hh, mid;
-  GBFEM_HD explicit FxAcc(long long start = 0, long long round = 0) : hh(start), mid(round) {}
+  bool no_hh, no_mid;
+  GBFEM_HD FxAcc() : hh(0), mid(0), no_hh(true), no_mid(true) {}
+  GBFEM_HD FxAcc(long long start, long long round) : hh(start), mid(round), no_hh(false), no_mid(false) {}
+  GBFEM_HD static FxAcc rounded() {
+    FxAcc r;
+    r.mid = 1ll << 31;
+    r.no_mid = false;
+    return r;
+  }
   GBFEM_HD void add(FxLimbs x, FxCoef c) {
-    hh += (long long)x.h * c.h;
-    mid += (long long)x.h * c.l;
-    mid += (long long)x.l * c.h;
+    hh = no_hh ? fx_mul(x.h, c.h) : fx_mad(x.h, c.h, hh);
+    mid = no_mid ? fx_mul(x.h, c.l) : fx_mad(x.h, c.l, mid);
+    mid = fx_mad(x.l, c.h, mid);
+    no_hh = no_mid = false;
   }
   GBFEM_HD long long value() const { return hh + (mid >> 32); }
   // the sum times 2^K, with K more of its digits

@@ -247,7 +247,7 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
       fill_line_operators(op, &ct);
       // One kernel over whole z-planes where the coefficients fit the fixed
       // point (fx_make_tables).  It has no trace pass: phase 1 only copies.
-      // 64^3 Q3: 319 us against 822 for the two FP64-pipe kernels, which stay
+      // 64^3 Q3: 295 us against 822 for the two FP64-pipe kernels, which stay
       // for a kappa per cell and refused coefficients.
       const long long plane = (long long)a.nc[0] * a.nc[1];
       const long long count = cell_count > 0 ? cell_count : op->ncells - cell_begin;

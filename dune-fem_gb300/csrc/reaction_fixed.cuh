@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(RxShape<N, Q>::T) dg_reaction_fixed_kernel(
       uint64_t any = 0;
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
-        FxAcc acc(0, 1ll << 31);
+        FxAcc acc = FxAcc::rounded();
 #pragma unroll
         for (int i = 0; i < N; ++i) acc.add(l[i], rx.B[q * N + i]);
         const double uq = double(acc.value()) * sScale[c];
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(RxShape<N, Q>::T) dg_reaction_fixed_kernel(
       uint32_t m = 0;
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        FxAcc acc(0, 1ll << 31);
+        FxAcc acc = FxAcc::rounded();
 #pragma unroll
         for (int q = 0; q < Q; ++q) acc.add(l[q], rx.BT[i * Q + q]);
         const long long t = acc.value();
@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(RxShape<N, Q>::T) dg_reaction_fixed_kernel(
     double* wc = w + (c0 + c) * N3 + jk;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      FxAcc acc(0, 1ll << 31);
+      FxAcc acc = FxAcc::rounded();
 #pragma unroll
       for (int a = 0; a < Q; ++a) acc.add(l[a], rx.BT[i * Q + a]);
       wc[i * N2] = fma(double(acc.value()), scale, wc[i * N2]);
