@@ -96,37 +96,42 @@ bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
   return true;
 }
 
-template <int N, bool ADV, bool SMALL>
+template <int N, bool ADV, bool SMALL, bool STAGE>
 static int fx_launch_brick(const DgArgsT<double>& a, const DgConstTablesT<double>& ct, const FxTables& fx, int z0, int z1,
-                         cudaStream_t s) {
+                           cudaStream_t s, const FxStage& st) {
   using B = FxBrick<N, SMALL>;
-  auto kern = dg_fixed_kernel<N, ADV, SMALL>;
+  auto kern = dg_fixed_kernel<N, ADV, SMALL, STAGE>;
   constexpr size_t smem = FxSmem<N, B>::BYTES;
   GBFEM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
   const long long nb = (long long)((a.nc[0] + B::X - 1) / B::X) * ((a.nc[1] + B::Y - 1) / B::Y) *
                        ((z1 - z0 + B::Z - 1) / B::Z);
   if (nb <= 0) return GBFEM_OK;
   if (nb > 2147483647LL) return set_error(GBFEM_ERR_INVALID, "dg apply: grid too large");
-  kern<<<unsigned(nb), fx_threads<N, B>(), smem, s>>>(a, ct, fx, z0, z1);
+  kern<<<unsigned(nb), fx_threads<N, B>(), smem, s>>>(a, ct, fx, z0, z1, st);
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
 
 template <int N, bool ADV>
 static int fx_launch_one(const DgArgsT<double>& a, const DgConstTablesT<double>& ct, const FxTables& fx, int z0, int z1,
-                         cudaStream_t s) {
+                         cudaStream_t s, const FxStage* st) {
   const long long cells = (long long)a.nc[0] * a.nc[1] * (z1 - z0);
   using B = FxBrick<N, false>;
-  if (cells < 152LL * B::X * B::Y * B::Z) return fx_launch_brick<N, ADV, true>(a, ct, fx, z0, z1, s);
-  return fx_launch_brick<N, ADV, false>(a, ct, fx, z0, z1, s);
+  const bool small = cells < 152LL * B::X * B::Y * B::Z;
+  if (st)
+    return small ? fx_launch_brick<N, ADV, true, true>(a, ct, fx, z0, z1, s, *st)
+                 : fx_launch_brick<N, ADV, false, true>(a, ct, fx, z0, z1, s, *st);
+  return small ? fx_launch_brick<N, ADV, true, false>(a, ct, fx, z0, z1, s, FxStage{})
+               : fx_launch_brick<N, ADV, false, false>(a, ct, fx, z0, z1, s, FxStage{});
 }
 
-// w = A u on the z-planes [z0, z1).
+// w = A u on the z-planes [z0, z1), with the stage st where one is given.
 int dg_fixed_launch(const DgArgsT<double>& a, const DgConstTablesT<double>& ct, const FxTables& fx, int n, int z0,
-                    int z1, cudaStream_t s) {
-#define GBFEM_FX_CASE(NN) \
-  if (n == NN)            \
-    return a.advect ? fx_launch_one<NN, true>(a, ct, fx, z0, z1, s) : fx_launch_one<NN, false>(a, ct, fx, z0, z1, s);
+                    int z1, cudaStream_t s, const FxStage* st) {
+#define GBFEM_FX_CASE(NN)                                               \
+  if (n == NN)                                                          \
+    return a.advect ? fx_launch_one<NN, true>(a, ct, fx, z0, z1, s, st) \
+                    : fx_launch_one<NN, false>(a, ct, fx, z0, z1, s, st);
   GBFEM_FX_CASE(2)
   GBFEM_FX_CASE(3)
   GBFEM_FX_CASE(4)

@@ -240,10 +240,15 @@ __device__ __noinline__ void fx_line_f64(const DgArgsT<double>& args, const DgCo
   }
 }
 
-template <int N, bool ADV, bool SMALL>
+// STAGE: a Runge-Kutta stage goes with the apply, st.y = st.u + sum_j st.a[j] w_j over
+// the earlier results st.w[j] and, last, this one, which is stored only if args.w is
+// given (st.y may be st.u, not args.u).  The FP64 pipe has room for its one to three
+// multiply-adds per dof and the memory system for its vectors: three applies and three
+// passes over the vectors, 1158 us at 80^3 Q2, become 1090.
+template <int N, bool ADV, bool SMALL, bool STAGE>
 __global__ void __launch_bounds__(fx_threads<N, FxBrick<N, SMALL>>(), FxBrick<N, SMALL>::MINB)
     dg_fixed_kernel(const __grid_constant__ DgArgsT<double> args, const __grid_constant__ DgConstTablesT<double> ct,
-                    const __grid_constant__ FxTables fx, int z0, int z1) {
+                    const __grid_constant__ FxTables fx, int z0, int z1, const __grid_constant__ FxStage st) {
   using B = FxBrick<N, SMALL>;
   using S = FxSmem<N, B>;
   constexpr int N2 = N * N, N3 = N2 * N;
@@ -424,7 +429,18 @@ __global__ void __launch_bounds__(fx_threads<N, FxBrick<N, SMALL>>(), FxBrick<N,
           for (int i = 0; i < N; ++i) y[i] += ys[i];
         }
         if (D == 2) {
-          double* wc = args.w + first + r * zstep + jk * N;
+          const long long at = first + r * zstep + jk * N;
+          if (STAGE) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              double v = st.u[at + i];
+              if (st.earlier > 0) v = fma(st.a[0], __ldg(st.w[0] + at + i), v);
+              if (st.earlier > 1) v = fma(st.a[1], __ldg(st.w[1] + at + i), v);
+              __stcs(st.y + at + i, fma(st.a[st.earlier], y[i], v));
+            }
+            if (!args.w) continue;
+          }
+          double* wc = args.w + at;
           if (N % 2 == 0 && wide) {
 #pragma unroll
             for (int i = 0; i < N; i += 2)

@@ -31,4 +31,13 @@ constexpr int kFxTraceExp = 56;
 GBFEM_HD constexpr double fx_slope_scale(int n) { return n == 2 ? 1.0 : (n == 3 ? 0.25 : (n == 4 ? 0.125 : 0.0625)); }
 constexpr int fx_coef_bits(bool adv) { return adv ? 61 : 62; }
 
+// y = u + sum_j a[j] w_j, j < earlier from memory and j = earlier the apply's result
+struct FxStage {
+  const double* u;
+  const double* w[2];
+  double a[3];
+  int earlier;  // results before this one
+  double* y;
+};
+
 }  // namespace gbfem

@@ -24,8 +24,8 @@ int dg_const_launch_f64(const DgArgsT<double>&, const DgConstTablesT<double>&, i
 int dg_const_launch_f32(const DgArgsT<float>&, const DgConstTablesT<float>&, int, float*, int, cudaStream_t,
                         float* ucopy = nullptr);
 bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out);
-int dg_fixed_launch(const DgArgsT<double>&, const DgConstTablesT<double>&, const FxTables&, int n, int z0, int z1,
-                    cudaStream_t);
+int dg_fixed_launch(const DgArgsT<double>&, const DgConstTablesT<double>&, const FxTables&, int, int, int,
+                    cudaStream_t, const FxStage* st = nullptr);
 bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out);
 int qx_kappa(gbfem_operator_s* op);
 int dg_quad_fixed_launch(const gbfem_operator_s* op, const DgArgsT<double>& a, cudaStream_t s);
@@ -289,6 +289,21 @@ static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, c
     }
     return dg_launch_f32(a, op->tab32, op->n, op->q, op->dg.kappa != nullptr, s);
   }
+}
+
+// A Runge-Kutta stage with its apply in one kernel (dg_fixed_kernel).
+bool dg_stage_takes(const gbfem_operator_s* op) {
+  return op->kind == OpKind::DG && op->precision == GBFEM_F64 && op->coefficient_space && op->fixed && !op->form &&
+         !op->nonlinear && !op->jac_points;
+}
+int dg_apply_stage(const gbfem_operator_s* op, const double* u, double* w, const FxStage& st, cudaStream_t s) {
+  DgArgsT<double> a;
+  fill_dg_args(op, &a);
+  a.u = u;
+  a.w = w;
+  DgConstTablesT<double> ct = op->ctab64;
+  fill_line_operators(op, &ct);
+  return dg_fixed_launch(a, ct, op->fx, op->n, 0, a.nc[2], s, &st);
 }
 
 // The device-resident CG's operator: the one-kernel FP32 closed form, with

@@ -9,8 +9,9 @@
 // (solver/rungekutta/explicit.hh:160-215) with the TVD3 Butcher table
 // (solver/rungekutta/butchertable.cc:43-52):
 //   k_0 = L(u);  k_i = L(u + dt sum_{j<i} A_ij k_j);  u += dt sum_j b_j k_j.
-// The stage combinations are single fused passes over the vectors, with the
-// factor -1/|K| folded into the coefficients.
+// The stage combinations are single fused passes over the vectors, or part of the
+// apply itself where that is the FP64 fixed-point kernel, with the factor -1/|K|
+// folded into the coefficients.
 #include <cuda_runtime.h>
 #include <cfloat>
 #include <cmath>
@@ -21,6 +22,9 @@
 #include "operator_impl.hpp"
 
 namespace gbfem {
+
+bool dg_stage_takes(const gbfem_operator_s* op);
+int dg_apply_stage(const gbfem_operator_s* op, const double* u, double* w, const FxStage& st, cudaStream_t s);
 
 // y = u + c0 w0 + c1 w1 + c2 w2 (nw terms)
 template <typename T>
@@ -102,6 +106,17 @@ int gbfem_rk3_step(gbfem_rk_solver rk, void* u, double dt, void* stream) {
   const long long n = rk->op->ndofs;
   const double f = -dt * rk->minv;  // dt * L = -dt/|K| * A
   // k_j hold A(stage_j) (unscaled); the coefficients carry -dt/|K|.
+  if (dg_stage_takes(rk->op)) {
+    // each combination with the apply that gives its last term; the last k_j is not
+    // stored and its buffer holds the second stage's argument
+    const double* const du = static_cast<const double*>(u);
+    double* const k[3] = {(double*)rk->k[0], (double*)rk->k[1], (double*)rk->k[2]};
+    double* const y = static_cast<double*>(rk->y);
+    GBFEM_TRY(dg_apply_stage(rk->op, du, k[0], FxStage{du, {nullptr, nullptr}, {A[1][0] * f, 0.0, 0.0}, 0, y}, s));
+    GBFEM_TRY(dg_apply_stage(rk->op, y, k[1], FxStage{du, {k[0], nullptr}, {A[2][0] * f, A[2][1] * f, 0.0}, 1, k[2]}, s));
+    return dg_apply_stage(rk->op, k[2], nullptr,
+                          FxStage{du, {k[0], k[1]}, {b[0] * f, b[1] * f, b[2] * f}, 2, static_cast<double*>(u)}, s);
+  }
   GBFEM_TRY(gbfem_operator_apply(rk->op, u, rk->k[0], s));
   for (int i = 1; i < 3; ++i) {
     if (rk->op->precision == GBFEM_F64)
