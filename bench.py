@@ -38,17 +38,13 @@ METRIC = "SIPG apply DoF/s"
 UNIT = "DoF/s"
 BYTES_PER_DOF = 16.0          # read u (8) + write w (8), geometry recomputed, tables on chip
 FLOP_PER_DOF = 402.0          # sum-factorised SIPG Q3, q=5 (volume + faces), the algorithmic count
-# flops the closed-form kernels execute per cell (n = 4, constant kappa, no
-# mass, no advection; an FMA counts 2), divided by n^3:
-#  traces: 3 n^2 lines x (even/odd partial sums of v and P: 4 FMA + 2 MUL,
-#          u_0 enters both even sums as is; 4 adds for the two faces) = 48 x 14
-#  fluxes: 6 n^2 face points x 2 (J = v- - v+, P- - P+)             = 96 x 2
-#  lines:  n^2 lines per axis x (4 adds + 2 x (5 structural nonzeros of M_d
-#          + 7 face-expansion FMAs))                                = 48 x 28
-KERNEL_FLOP_PER_DOF = (48 * 14 + 96 * 2 + 48 * (4 + 2 * (5 + 7))) / 64.0  # = 34.5
-# FP64 instructions per dof, which is what the FP64 pipe issues (an add takes
-# the slot of an FMA): (48 x 10 + 96 x 2 + 48 x 16) / 64
-KERNEL_FP64_INSTR_PER_DOF = (48 * 10 + 96 * 2 + 48 * 16) / 64.0  # = 22.5
+# What the headline kernel (dg_fixed_kernel: the closed form in 64-bit block fixed
+# point on the integer pipes) leaves to the FP64 pipe, per dof and axis: one integer
+# to double conversion and one fused multiply-add.
+KERNEL_FLOP_PER_DOF = 6.0
+KERNEL_FP64_INSTR_PER_DOF = 6.0
+# all instructions it executes per dof (counted by the profiler: 229.0M warp instructions)
+KERNEL_INSTR_PER_DOF = 437.0
 CONFIG = {"workload": "SIPG DG Q3 apply, 3-D unit cube 64^3 hexes, 16.8M dofs, q=5, penalty 160, FP64",
           "cells": list(CELLS), "order": ORDER, "quad_points": QUAD, "dofs": 64 ** 3 * 64,
           "l2": "inputs exceed L2 (u + w = 268 MB > 129 MB), no flush"}
@@ -296,15 +292,18 @@ def solve_comparison():
 
 
 def profiled_traffic(path):
-    """DRAM bytes of one headline apply from the committed ncu summary:
-    (both kernels: trace pass + main kernel, main kernel alone, launch-list
-    share of the main kernel), or (None, None, None) without the file."""
+    """DRAM bytes of one headline apply from a committed ncu summary: (the whole
+    apply, its main kernel alone, the main kernel's share of the launch list), or
+    (None, None, None) without the file.  A summary with a trace kernel is of the
+    two-kernel form, one without is of a single kernel."""
     if not os.path.exists(path):
         return None, None, None
     with open(path) as f:
         d = json.load(f)
     main = d.get("dram_bytes_per_launch")
     t = d.get("trace_kernel") or {}
+    if "trace_kernel" not in d:
+        return main, main, 1.0
     step = None
     if main is not None and "dram_read" in t and "dram_write" in t:
         step = int(main + t["dram_read"] + t["dram_write"])
@@ -404,7 +403,7 @@ def run_gpu(args, world, rank, local):
     achieved_gbs = BYTES_PER_DOF * n / (ms_step * 1e-3) / 1e9
     achieved_tflops = KERNEL_FLOP_PER_DOF * n / (ms_step * 1e-3) / 1e12
     traffic, traffic_main, main_share = profiled_traffic(
-        os.path.join(ROOT, "profiles", "dg_trace_const_q3_64cube_f64.json"))
+        os.path.join(ROOT, "profiles", "dg_fixed_q3_64cube_f64.json"))
     # CPU baseline: the oracle on this host's cores, bounded sample (~15 s)
     import oracle
     prob = oracle.DGProblem(CELLS, ORDER, quad_points=QUAD)
@@ -414,17 +413,17 @@ def run_gpu(args, world, rank, local):
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64", "data": "synthetic (seeded uniform[-1,1] dofs)",
             "config": CONFIG,
-            "gpu_launches": 2 * args.steps,
+            "gpu_launches": args.steps,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 8 * n, "d2h_bytes_per_step": 8 * n,
                     "steps": e2e_steps,
-                    "path": "gbfem_operator_apply_host (page-locked host buffers; copy in, trace pass, apply and "
+                    "path": "gbfem_operator_apply_host (page-locked host buffers; copy in, apply and "
                             "copy out pipelined over 16 z-slabs on four streams, replayed as one CUDA graph)",
                     "in_place_c2c_value": e2e_in_place},
             "roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved_gbs / peaks["hbm_gbs"], "traffic": traffic,
                          "peak_source": peak_kind, "algorithmic_bytes_per_dof": BYTES_PER_DOF,
-                         "scope": "one apply: trace pass + main kernel (achieved and traffic alike)",
-                         "main_kernel": {"name": "dg_const_kernel", "traffic": traffic_main,
+                         "scope": "one apply, which is one kernel (achieved and traffic alike)",
+                         "main_kernel": {"name": "dg_fixed_kernel", "traffic": traffic_main,
                                          "launch_list_share": main_share,
                                          "frac_at_share": (achieved_gbs / main_share / peaks["hbm_gbs"])
                                          if main_share else None}},
@@ -432,19 +431,22 @@ def run_gpu(args, world, rank, local):
                           "frac": achieved_tflops / fp64_peak if fp64_peak else None,
                           "kernel_flop_per_dof": KERNEL_FLOP_PER_DOF,
                           "kernel_fp64_instructions_per_dof": KERNEL_FP64_INSTR_PER_DOF,
+                          "kernel_instructions_per_dof": KERNEL_INSTR_PER_DOF,
+                          "note": "the products run on the integer pipes; what bounds the kernel is the issue of "
+                                  "instructions",
                           "issue_frac": (KERNEL_FP64_INSTR_PER_DOF * n / (ms_step * 1e-3) / 1e12) / (fp64_peak / 2)
                           if fp64_peak else None,
                           "sum_factorised_quadrature_flop_per_dof": FLOP_PER_DOF,
                           "fp32_peak_tflops_measured": fp32_peak},
             "algorithm": "constant-kappa closed form of the q=5 Gauss quadrature (exact for these integrands; "
-                         "trace pre-pass + 1-D stiffness along lines + identity tangential face mass); "
-                         "2 kernel launches per apply",
+                         "1-D stiffness along lines + identity tangential face mass) in 64-bit block fixed point; "
+                         "1 kernel launch per apply",
             "quadrature_kernel": {"value": n / (ms_quad * 1e-3), "unit": UNIT, "ms_per_step": ms_quad,
                                   "rel_max_diff_vs_default": quad_rel,
                                   "note": "sum-factorised evaluation at the 125 Gauss points (the variable-kappa path)"},
             "fp32_apply": {"value": n / (ms_f32 * 1e-3), "unit": UNIT, "ms_per_step": ms_f32,
                            "hbm_frac": 8.0 * n / (ms_f32 * 1e-3) / 1e9 / peaks["hbm_gbs"],
-                           "kernel": "dg_cell_kernel (one kernel, no trace buffer; 8 B/dof algorithmic)",
+                           "kernel": "dg_plane_kernel (one kernel, no trace buffer; 8 B/dof algorithmic)",
                            "two_kernel_ms_per_step": ms_f32_two},
             "cpu_baseline": {"value": cpu_rate, "unit": UNIT, "cores": nthreads, "kind": "port",
                              "sample": "%d cells (whole z-slabs) of the 64^3 grid applied by the oracle "
@@ -938,7 +940,7 @@ def workload_apply_f32(args):
     """The constant-coefficient FP32 apply (cells^3, Q_order) alone, --steps
     times after 3 warm-up applies, with no other GPU work: the command the
     kernel profiles under profiles/ are taken from.  --algorithm 0 is the
-    default (one kernel for p <= 3), 2 the two-kernel trace-pass form;
+    default (one kernel), 2 the two-kernel trace-pass form;
     --kappa-cell uses a seeded kappa per cell."""
     import gbfem
     import torch
@@ -962,9 +964,9 @@ def workload_apply_f32(args):
 
 def workload_scaled_bj(args):
     """The scaled shared-block Jacobi apply of the cellwise-kappa FP32
-    operator (cells^3, Q_order, seeded kappa per cell) on both engines of its
-    tile products: tcgen05 tensor cores (3xTF32) and FP32 FMA; --steps applies
-    after 3 warm-up applies, CUDA events."""
+    operator (cells^3, Q_order, seeded kappa per cell) on both engines: fast
+    diagonalisation (named "tensor": products of 1-D transforms) and the dense
+    blocks by FP32 FMA; --steps applies after 3 warm-up applies, CUDA events."""
     import gbfem
     import torch
     N, p = args.cells, args.order
@@ -1103,7 +1105,7 @@ def workload_mixed_solve(args):
     """The mixed arm of the headline line's solve object alone (64^3 Q3,
     kappa seed 1, f = 1, to ||f - A u|| / ||f|| <= 1e-10): FP64 FGMRES(30) on
     the full kappa around the FP32 inner CG (device-resident, graph chunks of
-    16) on the cellwise-kappa one-kernel apply with the tcgen05 scaled block
+    16) on the cellwise-kappa one-kernel apply with the scaled block
     Jacobi.  --max-outer bounds the outer iterations (a short window for
     kernel launch lists)."""
     import gbfem
