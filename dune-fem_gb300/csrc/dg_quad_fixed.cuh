@@ -6,7 +6,7 @@
 // What bounds it: integer issue and the barriers between the contractions (2.1
 // instructions a clock and SM), about 3600 instructions per dof at Q3 in place of 135
 // clocks of FP64 pipe.  Measured (GB300), dg_apply_kernel before, this after:
-// 45 x 38 x 33 Q3 2152 -> 620 us.
+// 45 x 38 x 33 Q3 2152 -> 571 us.
 //
 // Numbers.  All of a cell's values are integers v 2^(s-(E-1022)) of its exponent E
 // (its largest dof's), |integer| <= 2^60; a contraction with a matrix c of row sums
@@ -119,10 +119,15 @@ __device__ __noinline__ void qx_cell_f64(const DgArgsT<double>& args, const DgTa
   dg_apply_cells<double, N, Q, true, 1>(one, tabs, sm, cell);
 }
 
+// Cells and threads per CTA.  32 warps per SM in four CTAs hide each other's barriers:
+// 45 x 38 x 33 Q3 takes 571 us, 621 with three CTAs (80 registers), 567 with five,
+// 648 with half the cells and threads in eight, 634 with 320 threads in three; Q1, Q2
+// and Q4 1056, 742 and 596 us at 101 x 77 x 64, 61 x 52 x 47 and 33 x 30 x 31, against
+// 1243, 820 and 781 with five CTAs of 128 threads.
 template <int N, int Q>
 struct QxShape {
-  static constexpr int CPB = N == 2 ? 32 : (N == 3 ? 16 : (N == 4 ? 8 : 4));
-  static constexpr int T = N == 4 ? 256 : 128, MINB = N == 4 ? 3 : 5;
+  static constexpr int CPB = N == 2 ? 32 : (N == 3 ? 16 : (N == 4 ? 8 : 6));
+  static constexpr int T = 256, MINB = 4;
 };
 
 template <int N, int Q>

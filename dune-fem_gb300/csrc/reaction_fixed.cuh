@@ -29,8 +29,11 @@ struct RxTables {
 
 template <int N, int Q>
 struct RxShape {
-  static constexpr int CPB = N == 2 ? 32 : (N == 3 ? 16 : (N == 4 ? 8 : 4));
-  static constexpr int T = 128;
+  // Newton's three calls on 32^3 Q2 and 30 x 29 x 30 Q3: 170 and 304 us; with 16 cells
+  // at Q2 174, without the register bound (MINB) 331 at Q3, with 256 threads 176 and
+  // 305; 9 x 10 x 11 Q2 41 us, 50 with 16 cells.
+  static constexpr int CPB = N == 2 ? 32 : (N == 3 || N == 4 ? 8 : 4);
+  static constexpr int T = 128, MINB = N == 5 ? 1 : 8;
   static constexpr int N2 = N * N, N3 = N2 * N, Q2 = Q * Q, Q3 = Q2 * Q;
   static constexpr int WS = Q * N2 + Q2 * N;  // t1, t2
   static constexpr size_t BYTES = size_t(CPB) * (N3 + WS) * 8 + size_t(Q3) * 8 + 32 * 8;
@@ -44,7 +47,7 @@ __device__ __noinline__ void rx_cell_f64(int mode, const double* u, double* w, d
 
 // modes as dg_reaction_body
 template <int N, int Q, int MODE>
-__global__ void __launch_bounds__(RxShape<N, Q>::T) dg_reaction_fixed_kernel(
+__global__ void __launch_bounds__(RxShape<N, Q>::T, RxShape<N, Q>::MINB) dg_reaction_fixed_kernel(
     const double* __restrict__ u, double* __restrict__ w, double* __restrict__ pts, long long cell_begin,
     long long count, const __grid_constant__ ReactTabsT<double> tb, const __grid_constant__ RxTables rx) {
   using S = RxShape<N, Q>;
