@@ -220,6 +220,20 @@ __global__ void k_block_apply(const T* __restrict__ binvT, const T* __restrict__
   z[(c0 + lc) * nb + i] = acc;
 }
 
+// Cells per CTA of the FP64 kernel: the FP64 pipe binds (nb multiply-adds per dof at 2
+// per clock and SM) and also works for the idle lanes of a CTA's last warp, so the
+// count between 128 and 256 threads that leaves the fewest of them: nb = 27 (Q2) 7
+// cells in 6 warps, 2 % idle, 65.5 us for 47500 cells; 4 in 4 warps, 16 % idle, 73.8.
+static int block_cells_f64(int nb) {
+  const int lo = nb >= 128 ? 1 : 128 / nb, hi = nb >= 256 ? 1 : 256 / nb;
+  int best = lo;
+  for (int c = lo + 1; c <= hi; ++c) {
+    const int used = c * nb, all = (used + 31) / 32 * 32, used0 = best * nb, all0 = (used0 + 31) / 32 * 32;
+    if ((long long)used * all0 > (long long)used0 * all) best = c;
+  }
+  return best;
+}
+
 // Scaled shared-block Jacobi of an operator with a constant kappa per cell
 // (no mass, no advection): z_c = Hinv_t(c) r_c / kappa_c.  Hinv_t is the
 // inverse diagonal block of the kappa = 1 operator for the cell's boundary
@@ -508,7 +522,7 @@ int precond_apply(const gbfem_preconditioner_s* pc, const void* r, void* z, cuda
     case PcKind::BlockJacobi: {
       const int nb = pc->nloc;
       const long long nc = n / nb;
-      const int cpb = nb >= 128 ? 1 : 128 / nb;
+      const int cpb = pc->precision == GBFEM_F64 ? block_cells_f64(nb) : (nb >= 128 ? 1 : 128 / nb);
       const int threads = ((cpb * nb + 31) / 32) * 32;
       const size_t sm = size_t(cpb) * nb * (pc->precision == GBFEM_F64 ? 8 : 4);
       const unsigned blocks = unsigned((nc + cpb - 1) / cpb);
