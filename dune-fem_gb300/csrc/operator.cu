@@ -231,6 +231,25 @@ __global__ void k_copy_dofs(long long n, const double* __restrict__ u, double* _
     v[i] = __ldg(u + i);
 }
 
+// *out: op as the mixed solve applies it (gbfem_solve_mixed), FP64 products on the FP64
+// pipe and FP32 ones of p = 4 in the two-kernel form; *keep holds a copy where that is
+// another form than op's own.  The copy shares all that op owns (the trace buffer is made
+// here, so that it is op's own).
+int dg_mixed_form(gbfem_operator_s* op, gbfem_operator_s* keep, gbfem_operator_s** out) {
+  *out = op;
+  const bool two = op->precision == GBFEM_F32 && op->coefficient_space && op->n == 5 && !op->two_kernel_f32;
+  if (!op->fixed && !op->quad_fixed && !two) return GBFEM_OK;
+  if (op->coefficient_space) {
+    void* tb = nullptr;
+    GBFEM_TRY(trace_buffer(op, &tb));
+  }
+  *keep = *op;
+  keep->fixed = keep->quad_fixed = false;
+  keep->two_kernel_f32 = two;
+  *out = keep;
+  return GBFEM_OK;
+}
+
 static int dg_apply_linear(const gbfem_operator_s* op, const void* u, void* w, cudaStream_t s, int unit_mode,
                            void* blocks, long long cell_begin, long long cell_count, int phase, void* ucopy) {
   if (op->precision == GBFEM_F64) {

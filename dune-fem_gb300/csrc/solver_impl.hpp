@@ -28,6 +28,7 @@ int sb_fdm_cg(const struct ::gbfem_preconditioner_s* pc, const void* q, const vo
 long long cg_apply_dot_parts(const struct ::gbfem_operator_s* op);
 int cg_apply_dot(const struct ::gbfem_operator_s* op, const void* q, void* h, double* partial, CgScalars* sc,
                  cudaStream_t s);
+int dg_mixed_form(struct ::gbfem_operator_s* op, struct ::gbfem_operator_s* keep, struct ::gbfem_operator_s** out);
 // the Q1 operator's CG in one kernel (q1_cg.cu), for the solves it takes
 bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
