@@ -301,6 +301,9 @@ static void sb_eigen(int n, long double (&a)[kDgMaxN][kDgMaxN], long double (&V)
   }
 }
 
+// The tables, in pc->sb_fdm; left null where a block is singular to FP32 rounding (one
+// cell without a boundary term: the division gives infinities, the dense inverse of
+// the rounded block does not).
 int sb_fdm_setup(gbfem_preconditioner_s* pc) {
   const gbfem_operator_s* op = pc->sor_op;
   const gbfem_dg_desc& d = op->dg;
@@ -308,7 +311,6 @@ int sb_fdm_setup(gbfem_preconditioner_s* pc) {
   const ConstTables1D ct = make_const_tables(n);
   auto* t = new (std::nothrow) SbFdmTables{};
   if (!t) return set_error(GBFEM_ERR_INVALID, "out of host memory");
-  pc->sb_fdm = t;
   long double h[3], vol = 1.0L, v[2][kDgMaxN], g[2][kDgMaxN];
   for (int k = 0; k < 3; ++k) {
     h[k] = ((long double)d.grid.upper[k] - d.grid.lower[k]) / d.grid.cells[k];
@@ -338,6 +340,26 @@ int sb_fdm_setup(gbfem_preconditioner_s* pc) {
         for (int j = 0; j < n; ++j) t->V[k][type][i * n + j] = float(V[i][j]);
       }
     }
+  // the boundary types that occur on an axis
+  auto occurs = [&](int k, int type) {
+    const int nc = d.grid.cells[k];
+    if (d.grid.periodic[k]) return type == 0;
+    return nc == 1 ? type == 3 : (type == 1 || type == 2 || (type == 0 && nc > 2));
+  };
+  bool regular = true;
+  for (int e = 0; e < 64; ++e) {
+    const int ty[3] = {e & 3, (e >> 2) & 3, e >> 4};
+    if (!occurs(0, ty[0]) || !occurs(1, ty[1]) || !occurs(2, ty[2])) continue;
+    float least = INFINITY, most = 0.f;
+    for (int l = 0; l < n * n * n; ++l) {
+      const float v = fabsf(t->L[0][ty[0]][l / (n * n)] + t->L[1][ty[1]][(l / n) % n] + t->L[2][ty[2]][l % n]);
+      least = fminf(least, v);
+      most = fmaxf(most, v);
+    }
+    regular = regular && least > 1e-6f * most;
+  }
+  if (regular) pc->sb_fdm = t;
+  else delete t;
   return GBFEM_OK;
 }
 

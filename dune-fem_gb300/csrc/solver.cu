@@ -1406,22 +1406,6 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
   if (op->kind != OpKind::DG || !d.kappa_cell || op->precision != GBFEM_F32 || d.mass != 0.0 || op->nonlinear)
     return set_error(GBFEM_ERR_INVALID,
                      "scaled block Jacobi: needs an FP32 DG operator with kappa_cell, no mass, not nonlinear");
-  if (engine == GBFEM_SB_ENGINE_TENSOR) {
-    auto* pc = new (std::nothrow) gbfem_preconditioner_s();
-    if (!pc) return set_error(GBFEM_ERR_INVALID, "out of host memory");
-    pc->kind = PcKind::ScaledBlock;
-    pc->precision = GBFEM_F32;
-    pc->n = op->ndofs;
-    pc->nloc = op->nloc;
-    pc->sor_op = op;
-    const int rc = sb_fdm_setup(pc);
-    if (rc) {
-      gbfem_preconditioner_destroy(pc);
-      return rc;
-    }
-    *out = pc;
-    return GBFEM_OK;
-  }
   // the kappa = 1 operator on a grid with one cell per boundary type, same cell size
   gbfem_dg_desc t = d;
   t.kappa = nullptr;
@@ -1453,6 +1437,13 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
   pc->data = tbj->data;  // take over the inverted type blocks
   tbj->data = nullptr;
   gbfem_preconditioner_destroy(tbj);
+  if (engine == GBFEM_SB_ENGINE_TENSOR) {  // (a singular block has been refused above)
+    const int rc = sb_fdm_setup(pc);
+    if (rc) {
+      gbfem_preconditioner_destroy(pc);
+      return rc;
+    }
+  }
   if (op->nloc > 32 && op->nloc <= 128) {
     // cells sorted by boundary type (stable: interior runs stay consecutive), tiles of <= 32
     const int* nc = d.grid.cells;

@@ -29,3 +29,32 @@ def test_against_dense_inverse(gb, orc, order, cells, kw):
     err = np.max(np.abs(z.numpy().reshape(nc, nloc) - ref), axis=1) / np.max(np.abs(ref), axis=1)
     assert np.all(err <= 40 * 2.0 ** -24 * np.linalg.cond(blocks))
     assert np.sqrt(np.mean(err ** 2)) < 2e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("engine", ["tensor", "fma"])
+def test_singular_blocks_are_refused(gb, engine):
+    """No diffusion: the blocks are zero."""
+    op = gb.DGOperator((3, 2, 1), 2, precision=gb.F32, diffusion=0.0,
+                       kappa_cell=gb.DeviceArray.from_numpy(np.ones(6, np.float32)))
+    with pytest.raises(gb.GbfemError):
+        gb.Preconditioner.scaled_block_jacobi(op, engine=engine)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2])
+def test_block_singular_up_to_rounding(gb, order):
+    """One cell whose constants nothing holds: the dense inverse of the rounded
+    block, with either engine."""
+    op = gb.DGOperator((1, 1, 1), order, precision=gb.F32, weak_dirichlet=False,
+                       kappa_cell=gb.DeviceArray.from_numpy(np.ones(1, np.float32)))
+    r = gb.DeviceArray.from_numpy(np.random.default_rng(1).uniform(-1, 1, op.size).astype(np.float32))
+    out = []
+    for engine in ("tensor", "fma"):
+        z = gb.DeviceArray(op.size, gb.F32)
+        try:
+            gb.Preconditioner.scaled_block_jacobi(op, engine=engine)(r, z)
+            out.append(z.numpy().view(np.uint32).tolist())
+        except gb.GbfemError as e:
+            out.append(str(e))
+    assert out[0] == out[1]
