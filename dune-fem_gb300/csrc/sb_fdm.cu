@@ -25,7 +25,6 @@
 #include <cmath>
 #include <new>
 
-#include "cg_device.cuh"
 #include "gbfem_internal.cuh"
 #include "operator_impl.hpp"
 #include "solver_impl.hpp"
@@ -39,15 +38,9 @@ struct SbFdmTables {
   float L[3][4][kDgMaxN];
 };
 
-// CG: one iteration's end (cg_device.cuh).  r is p, updated to p - alpha h before
-// the preconditioner takes it; x += alpha q; then <p, z> and the scalars.
 struct SbFdmArgs {
   const float *kcell, *r;
   float* z;
-  const float *q, *h;
-  float *x, *p;
-  double* partial;
-  CgScalars* sc;
   long long ncells;
   int nc[3], periodic[3];
 };
@@ -85,7 +78,7 @@ __device__ __forceinline__ void sb_plane(float (&x)[N * N], const float* __restr
   }
 }
 
-template <int N, bool CG>
+template <int N>
 __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ SbFdmArgs g,
                                                         const __grid_constant__ SbFdmTables tabs) {
   using S = SbFdm<N>;
@@ -94,8 +87,6 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   __shared__ float sV[3 * 4 * N2];
   __shared__ float sL[3 * 4 * N];
   __shared__ float sInv[N3];  // 1 / (Lx + Ly + Lz) of an interior cell, [i0][i1][i2]
-  if (CG && !g.sc->active) return;
-  const float alpha = CG ? g.sc->alpha_f : 0.f, minus = -alpha;
   const int tid = threadIdx.x;
   const long long c0 = (long long)blockIdx.x * S::CPB;
   const int ncell = int(g.ncells - c0 < S::CPB ? g.ncells - c0 : S::CPB);
@@ -109,53 +100,20 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   const float* rg = g.r + c0 * N3;
   float* zg = g.z + c0 * N3;
   const int total = ncell * N3;
-  const long long e0 = c0 * N3;
-  uintptr_t at = reinterpret_cast<uintptr_t>(rg) | reinterpret_cast<uintptr_t>(zg);
-  if (CG) at |= reinterpret_cast<uintptr_t>(g.q + e0) | reinterpret_cast<uintptr_t>(g.h + e0) |
-                reinterpret_cast<uintptr_t>(g.x + e0);
-  const bool wide = (at & 15) == 0 && total % 4 == 0;
+  const bool wide =
+      ((reinterpret_cast<uintptr_t>(rg) | reinterpret_cast<uintptr_t>(zg)) & 15) == 0 && total % 4 == 0;
   auto place = [](int e) { return N2 == PL ? e : (e / N2) * PL + e % N2; };
   constexpr int K4 = (N2 + 3) / 4;
-  float4 t[K4];  // CG: this thread's p, for <p, z>
   if (wide) {
+    float4 t[K4];
 #pragma unroll
     for (int j = 0; j < K4; ++j)
-      if (4 * (tid + j * T) < total)
-        t[j] = CG ? reinterpret_cast<const float4*>(rg)[tid + j * T] : __ldg(reinterpret_cast<const float4*>(rg) + tid + j * T);
-    if constexpr (CG) {
-#pragma unroll
-      for (int j = 0; j < K4; ++j) {
-        const int v = tid + j * T;
-        if (4 * v < total) {
-          const float4 h = __ldg(reinterpret_cast<const float4*>(g.h + e0) + v);
-          const float4 q = __ldg(reinterpret_cast<const float4*>(g.q + e0) + v);
-          float4 x = reinterpret_cast<const float4*>(g.x + e0)[v];
-          x.x = alpha * q.x + x.x;
-          x.y = alpha * q.y + x.y;
-          x.z = alpha * q.z + x.z;
-          x.w = alpha * q.w + x.w;
-          reinterpret_cast<float4*>(g.x + e0)[v] = x;
-          t[j].x = minus * h.x + t[j].x;
-          t[j].y = minus * h.y + t[j].y;
-          t[j].z = minus * h.z + t[j].z;
-          t[j].w = minus * h.w + t[j].w;
-          reinterpret_cast<float4*>(g.p + e0)[v] = t[j];
-        }
-      }
-    }
+      if (4 * (tid + j * T) < total) t[j] = __ldg(reinterpret_cast<const float4*>(rg) + tid + j * T);
 #pragma unroll
     for (int j = 0; j < K4; ++j)
       if (4 * (tid + j * T) < total) *reinterpret_cast<float4*>(buf + place(4 * (tid + j * T))) = t[j];
   } else {
-    for (int e = tid; e < total; e += T) {
-      float v = CG ? rg[e] : __ldg(rg + e);
-      if constexpr (CG) {
-        g.x[e0 + e] = alpha * g.q[e0 + e] + g.x[e0 + e];
-        v = minus * g.h[e0 + e] + v;
-        g.p[e0 + e] = v;
-      }
-      buf[place(e)] = v;
-    }
+    for (int e = tid; e < total; e += T) buf[place(e)] = __ldg(rg + e);
   }
   // this thread's cell and its type on each axis
   const int lc = tid / N, i = tid - lc * N;
@@ -238,62 +196,45 @@ __global__ void __launch_bounds__(SbFdm<N>::T) k_sb_fdm(const __grid_constant__ 
   else sb_plane<N, 1, false>(x, sV + (8 + type[2]) * N2);
   write_plane();
   __syncthreads();
-  DotAcc<float> acc;
   if (wide) {
 #pragma unroll
     for (int j = 0; j < K4; ++j)
-      if (4 * (tid + j * T) < total) {
-        const float4 v = *reinterpret_cast<const float4*>(buf + place(4 * (tid + j * T)));
-        reinterpret_cast<float4*>(zg)[tid + j * T] = v;
-        if (CG) {
-          acc.add(t[j].x, v.x);
-          acc.add(t[j].y, v.y);
-          acc.add(t[j].z, v.z);
-          acc.add(t[j].w, v.w);
-        }
-      }
+      if (4 * (tid + j * T) < total)
+        reinterpret_cast<float4*>(zg)[tid + j * T] = *reinterpret_cast<const float4*>(buf + place(4 * (tid + j * T)));
   } else {
-    for (int e = tid; e < total; e += T) {
-      const float v = buf[place(e)];
-      zg[e] = v;
-      if (CG) acc.add(g.p[e0 + e], v);
-    }
-  }
-  if constexpr (CG) {
-    if (!cg_deliver(cg_block_part(acc), g.partial, g.sc, 1)) return;
-    const double sum = cg_sum_parts(g.partial, int(gridDim.x));
-    if (tid == 0) cg_set_end(g.sc, sum);
+    for (int e = tid; e < total; e += T) zg[e] = buf[place(e)];
   }
 }
 
 // Eigenvectors (columns of V) and values of the symmetric n x n matrix a, by
-// cyclic Jacobi rotations (Golub & Van Loan, section 8.5).
-static void sb_eigen(int n, long double (&a)[kDgMaxN][kDgMaxN], long double (&V)[kDgMaxN][kDgMaxN]) {
+// cyclic Jacobi rotations (Golub & Van Loan, section 8.5).  In double: the tables are
+// FP32, and extended precision is slow on hosts that emulate it.
+static void sb_eigen(int n, double (&a)[kDgMaxN][kDgMaxN], double (&V)[kDgMaxN][kDgMaxN]) {
   for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) V[i][j] = i == j ? 1.0L : 0.0L;
+    for (int j = 0; j < n; ++j) V[i][j] = i == j ? 1.0 : 0.0;
   for (int sweep = 0; sweep < 30; ++sweep) {
-    long double off = 0.0L, dia = 0.0L;
+    double off = 0.0, dia = 0.0;
     for (int i = 0; i < n; ++i)
       for (int j = 0; j < n; ++j) (i == j ? dia : off) += a[i][j] * a[i][j];
-    if (!(off > 1e-38L * dia)) break;
+    if (!(off > 1e-30 * dia)) break;
     for (int p = 0; p < n; ++p)
       for (int q = p + 1; q < n; ++q) {
-        if (a[p][q] == 0.0L) continue;
-        const long double tau = (a[q][q] - a[p][p]) / (2.0L * a[p][q]);
-        const long double t = (tau >= 0.0L ? 1.0L : -1.0L) / (fabsl(tau) + sqrtl(1.0L + tau * tau));
-        const long double c = 1.0L / sqrtl(1.0L + t * t), s = t * c;
+        if (a[p][q] == 0.0) continue;
+        const double tau = (a[q][q] - a[p][p]) / (2.0 * a[p][q]);
+        const double t = (tau >= 0.0 ? 1.0 : -1.0) / (std::fabs(tau) + std::sqrt(1.0 + tau * tau));
+        const double c = 1.0 / std::sqrt(1.0 + t * t), s = t * c;
         for (int k = 0; k < n; ++k) {
-          const long double x = a[k][p], y = a[k][q];
+          const double x = a[k][p], y = a[k][q];
           a[k][p] = c * x - s * y;
           a[k][q] = s * x + c * y;
         }
         for (int k = 0; k < n; ++k) {
-          const long double x = a[p][k], y = a[q][k];
+          const double x = a[p][k], y = a[q][k];
           a[p][k] = c * x - s * y;
           a[q][k] = s * x + c * y;
         }
         for (int k = 0; k < n; ++k) {
-          const long double x = V[k][p], y = V[k][q];
+          const double x = V[k][p], y = V[k][q];
           V[k][p] = c * x - s * y;
           V[k][q] = s * x + c * y;
         }
@@ -321,7 +262,7 @@ int sb_fdm_setup(gbfem_preconditioner_s* pc) {
   for (int k = 0; k < 3; ++k)
     for (int type = 0; type < 4; ++type) {
       const long double eps = d.diffusion, area = vol / h[k], sigma = d.penalty / h[k];
-      long double a[kDgMaxN][kDgMaxN], V[kDgMaxN][kDgMaxN];
+      double a[kDgMaxN][kDgMaxN], V[kDgMaxN][kDgMaxN];
       for (int i = 0; i < n; ++i)
         for (int j = 0; j < n; ++j) {
           long double m = eps * vol / (h[k] * h[k]) * ct.K1[i][j];
@@ -332,7 +273,7 @@ int sb_fdm_setup(gbfem_preconditioner_s* pc) {
             const long double w = edge ? 1.0L : 0.5L, sg = s ? 1.0L / h[k] : -1.0L / h[k];
             m += eps * area * (sigma * v[s][i] * v[s][j] - w * sg * (g[s][i] * v[s][j] + v[s][i] * g[s][j]));
           }
-          a[i][j] = m;
+          a[i][j] = double(m);
         }
       sb_eigen(n, a, V);
       for (int i = 0; i < n; ++i) {
@@ -371,14 +312,16 @@ static int sb_fdm_launch(const SbFdmArgs& a, const SbFdmTables& t, cudaStream_t 
   const long long grid = (a.ncells + S::CPB - 1) / S::CPB;
   if (grid <= 0) return GBFEM_OK;
   if (grid > 2147483647LL) return set_error(GBFEM_ERR_INVALID, "scaled block Jacobi: grid too large");
-  if (a.sc) k_sb_fdm<N, true><<<unsigned(grid), S::T, 0, s>>>(a, t);
-  else k_sb_fdm<N, false><<<unsigned(grid), S::T, 0, s>>>(a, t);
+  k_sb_fdm<N><<<unsigned(grid), S::T, 0, s>>>(a, t);
   GBFEM_CUDA_TRY(cudaGetLastError());
   return GBFEM_OK;
 }
 
-static int sb_fdm_run(const gbfem_preconditioner_s* pc, SbFdmArgs& a, cudaStream_t s) {
+int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s) {
   const gbfem_operator_s* op = pc->sor_op;
+  SbFdmArgs a{};
+  a.r = r;
+  a.z = z;
   a.kcell = static_cast<const float*>(op->dg.kappa_cell);
   a.ncells = op->ncells;
   for (int d = 0; d < 3; ++d) {
@@ -393,34 +336,6 @@ static int sb_fdm_run(const gbfem_preconditioner_s* pc, SbFdmArgs& a, cudaStream
     case 5: return sb_fdm_launch<5>(a, t, s);
   }
   return set_error(GBFEM_ERR_NOT_IMPLEMENTED, "scaled block Jacobi: unsupported order");
-}
-
-int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s) {
-  SbFdmArgs a{};
-  a.r = r;
-  a.z = z;
-  return sb_fdm_run(pc, a, s);
-}
-
-long long sb_fdm_cg_parts(const gbfem_preconditioner_s* pc) {
-  if (pc->kind != PcKind::ScaledBlock || !pc->sb_fdm) return 0;
-  const int n = pc->sor_op->n;
-  const int cpb = n == 2 ? SbFdm<2>::CPB : (n == 3 ? SbFdm<3>::CPB : (n == 4 ? SbFdm<4>::CPB : SbFdm<5>::CPB));
-  return (pc->sor_op->ncells + cpb - 1) / cpb;
-}
-
-int sb_fdm_cg(const gbfem_preconditioner_s* pc, const void* q, const void* h, void* x, void* p, void* s_out,
-              double* partial, CgScalars* sc, cudaStream_t s) {
-  SbFdmArgs a{};
-  a.r = static_cast<const float*>(p);
-  a.z = static_cast<float*>(s_out);
-  a.q = static_cast<const float*>(q);
-  a.h = static_cast<const float*>(h);
-  a.x = static_cast<float*>(x);
-  a.p = static_cast<float*>(p);
-  a.partial = partial;
-  a.sc = sc;
-  return sb_fdm_run(pc, a, s);
 }
 
 }  // namespace gbfem

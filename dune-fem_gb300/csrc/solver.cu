@@ -556,8 +556,8 @@ int precond_apply(const gbfem_preconditioner_s* pc, const void* r, void* z, cuda
         g.nc[d] = pc->sor_op->dg.grid.cells[d];
         g.per[d] = pc->sor_op->dg.grid.periodic[d];
       }
-      if (pc->sb_fdm) {
-        return sb_fdm_apply(pc, (const float*)r, (float*)z, s);
+      if (pc->sb_tc_tiles) {
+        return sb_tc_apply(pc, (const float*)pc->sor_op->dg.kappa_cell, (const float*)r, (float*)z, s);
       } else if (pc->sb_tiles) {
         // one CTA per SM over a contiguous range of quads: the inverse and
         // two residual tiles per group, 192 KB at nb = 125
@@ -668,8 +668,10 @@ static int cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_par
 // instead of synchronising on every scalar product.  The scalar products end in
 // their last CTA, which also does the scalar statement that follows (alpha; the
 // end of the iteration and beta): no single-CTA kernels in between.  Divisions
-// and updates are the host loop's, so the iterates are identical -- except with
-// the scaled block Jacobi, whose fused kernels sum in their own order.
+// and updates are the host loop's, so the iterates are identical -- but for the
+// one-kernel FP32 products (cg_apply_dot), whose CTAs sum <q, h> over their own
+// cells: compensated sums that differ in the last bits of FP64, and alpha, rounded to
+// FP32, almost never.
 
 // q = s + beta q with a preconditioner, p = beta p - r without
 template <typename T>
@@ -806,15 +808,12 @@ static int cg_device(gbfem_operator op, gbfem_preconditioner pc, const gbfem_sol
   CgDeviceState& w = keep ? *keep : own;
   const long long n = c.n;
   const int np = dot_num_partials(n);
-  // fused kernels: the whole-grid FP32 closed form with <q, h>, and the update
-  // with the scaled block Jacobi and <p, s>
+  // the whole-grid FP32 closed form has <q, h> in its end
   const bool fuse_apply = cg_apply_dot_parts(op) > 0;
-  const bool fuse_pc = pc && sb_fdm_cg_parts(pc) > 0;
   if (!w.sc) {
     GBFEM_TRY(w.tmp.alloc(pc ? 5 : 3, c.bytes()));
     long long parts = np;
     if (fuse_apply) parts = std::max<long long>(parts, cg_apply_dot_parts(op));
-    if (fuse_pc) parts = std::max<long long>(parts, sb_fdm_cg_parts(pc));
     GBFEM_CUDA_TRY(cudaMalloc(&w.partial, sizeof(double) * size_t(parts)));
     GBFEM_CUDA_TRY(cudaMalloc(&w.sc, sizeof(CgScalars)));
   }
@@ -872,7 +871,6 @@ static int cg_device(gbfem_operator op, gbfem_preconditioner pc, const gbfem_sol
       else
         k_cg_dot<float, 0><<<np, kRedThreads, 0, st>>>(n, dchunk, (const float*)q, (const float*)h, partial, sc);
     }
-    if (fuse_pc) return sb_fdm_cg(pc, q, h, x, p, s, partial, sc, st);
     void* v = pc ? p : r;
     const int mode = !pc ? 0 : (diag_pc ? 1 : 2);
 #define GBFEM_CG_UPDATE(TT, M)                                                                                 \
@@ -1393,7 +1391,11 @@ int gbfem_preconditioner_scaled_block_jacobi_create(gbfem_operator op, gbfem_pre
 
 int gbfem_preconditioner_status(gbfem_preconditioner pc, int* status) {
   if (!pc || !status) return set_error(GBFEM_ERR_INVALID, "gbfem_preconditioner_status: null argument");
-  *status = 0;  // no preconditioner kernel has a wait that can give up
+  *status = 0;
+  if (pc->sb_tc_status) {
+    GBFEM_CUDA_TRY(cudaDeviceSynchronize());
+    GBFEM_CUDA_TRY(cudaMemcpy(status, pc->sb_tc_status, sizeof(int), cudaMemcpyDeviceToHost));
+  }
   return GBFEM_OK;
 }
 
@@ -1490,6 +1492,13 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
       return set_cuda_error(e, "scaled block Jacobi: tiles");
     }
     pc->sb_ntiles = (long long)(tiles.size() / 3);
+    if (engine == GBFEM_SB_ENGINE_TENSOR) {
+      const int rc = sb_tc_setup(pc, tiles, op->nloc, 0);
+      if (rc) {
+        gbfem_preconditioner_destroy(pc);
+        return rc;
+      }
+    }
   }
   *out = pc;
   return GBFEM_OK;
@@ -1497,6 +1506,13 @@ int gbfem_preconditioner_scaled_block_jacobi_create_engine(gbfem_operator op, in
 
 int gbfem_preconditioner_apply(gbfem_preconditioner pc, const void* r, void* z, void* stream) {
   if (!pc || !r || !z) return set_error(GBFEM_ERR_INVALID, "gbfem_preconditioner_apply: null argument");
+  // The scaled block Jacobi has two forms.  A direct apply takes the fast
+  // diagonalisation (48^3 Q4 44 us, the dense products 94; error against 64 bits 1.4e-7,
+  // 9e-7).  The solves keep the dense products: an FP32 CG amplifies a change of its
+  // preconditioner's rounding, and a mixed solve that stagnates then ends elsewhere
+  // (5e-5 to 7e-4 away on 495 and 1080 cells of Q2).
+  if (pc->sb_fdm) return sb_fdm_apply(pc, static_cast<const float*>(r), static_cast<float*>(z),
+                                      static_cast<cudaStream_t>(stream));
   return precond_apply(pc, r, z, static_cast<cudaStream_t>(stream));
 }
 
@@ -1512,6 +1528,9 @@ int gbfem_preconditioner_destroy(gbfem_preconditioner pc) {
   if (pc->scales) cudaFree(pc->scales);
   if (pc->sor_cells) cudaFree(pc->sor_cells);
   if (pc->sb_tiles) cudaFree(pc->sb_tiles);
+  if (pc->sb_tc_tiles) cudaFree(pc->sb_tc_tiles);
+  if (pc->sb_tc_img) cudaFree(pc->sb_tc_img);
+  if (pc->sb_tc_status) cudaFree(pc->sb_tc_status);
   if (pc->sb_fdm) sb_fdm_destroy(pc->sb_fdm);
   if (pc->sor_tmp) cudaFree(pc->sor_tmp);
   if (pc->ext_destroy) pc->ext_destroy(pc->ext_ctx);

@@ -13,17 +13,16 @@ enum class PcKind { Diagonal = 1, BlockJacobi = 2, External = 3, Sor = 4, Scaled
 int precond_apply(const struct ::gbfem_preconditioner_s* pc, const void* r, void* z, cudaStream_t s);
 // Jacobi / Gauss-Seidel / SOR / SSOR sweeps over an assembled operator (sor.cu)
 int sor_apply(const struct ::gbfem_preconditioner_s* pc, const void* r, void* z, cudaStream_t s);
-// scaled block Jacobi by fast diagonalisation (sb_fdm.cu)
+// scaled block Jacobi on the tensor cores (sb_tc.cu), the solves' form: set-up from
+// the (type, start, count) tiles, and the apply
+int sb_tc_setup(struct ::gbfem_preconditioner_s* pc, const std::vector<int>& tiles3, int nb, cudaStream_t s);
+int sb_tc_apply(const struct ::gbfem_preconditioner_s* pc, const float* kcell, const float* r, float* z,
+                cudaStream_t s);
+// the same by fast diagonalisation (sb_fdm.cu), the direct apply's form
 int sb_fdm_setup(struct ::gbfem_preconditioner_s* pc);
 int sb_fdm_apply(const struct ::gbfem_preconditioner_s* pc, const float* r, float* z, cudaStream_t s);
 void sb_fdm_destroy(void* tables);
 struct CgScalars;
-// the fused kernels of the device-resident CG: x += alpha q, p -= alpha h, s = P p,
-// <p, s> and the end of the iteration; the number of CTAs (parts), 0 where the
-// preconditioner is another one
-long long sb_fdm_cg_parts(const struct ::gbfem_preconditioner_s* pc);
-int sb_fdm_cg(const struct ::gbfem_preconditioner_s* pc, const void* q, const void* h, void* x, void* p, void* s_out,
-              double* partial, CgScalars* sc, cudaStream_t s);
 // h = A q, <q, h> and alpha; 0 parts where the operator has no such kernel
 long long cg_apply_dot_parts(const struct ::gbfem_operator_s* op);
 int cg_apply_dot(const struct ::gbfem_operator_s* op, const void* q, void* h, double* partial, CgScalars* sc,
@@ -61,9 +60,16 @@ struct gbfem_preconditioner_s {
   int* sor_cells = nullptr;
   void* sor_tmp = nullptr;
   std::vector<long long> sor_level_offsets;
-  // ScaledBlock by dense tiles: sor_cells holds the cells sorted by boundary type; tiles of
+  // ScaledBlock: sor_cells holds the cells sorted by boundary type; tiles of
   // (type, start, count) into it
   int* sb_tiles = nullptr;
   long long sb_ntiles = 0;
-  void* sb_fdm = nullptr;  // ScaledBlock by fast diagonalisation: its tables (host)
+  // ScaledBlock on the tensor cores: tiles without padding, A_hi | A_lo
+  // images per type, the kernel's status word (1 = a wait timed out)
+  int* sb_tc_tiles = nullptr;
+  int sb_tc_ntiles = 0;
+  int sb_tc_wide = 0;  // 64-cell tiles with K = 64 (blocks of up to 64 dofs)
+  void* sb_tc_img = nullptr;
+  int* sb_tc_status = nullptr;
+  void* sb_fdm = nullptr;  // ScaledBlock by fast diagonalisation: its tables (host), null without
 };

@@ -619,15 +619,16 @@ class Preconditioner:
     def scaled_block_jacobi(cls, op, engine="tensor"):
         """For an FP32 operator with kappa_cell (no mass): z_c = H_t^-1 r_c / kappa_c
         with the shared kappa = 1 blocks H_t of the cell's boundary type.
-        engine: "tensor" (the tensor-product form, by fast diagonalisation) or
-        "fma" (products with the dense inverses)."""
+        engine: "tensor" (applied directly by fast diagonalisation; in solves as
+        products with the dense inverses, on the tensor cores for p = 3, 4) or "fma"
+        (the dense inverses throughout, FP32 FMA)."""
         h = C.c_void_p()
         eng = {"tensor": 0, "fma": 1}[engine]
         check(lib().gbfem_preconditioner_scaled_block_jacobi_create_engine(op.handle, eng, C.byref(h)))
         return cls(h, F32, op)
 
     def status(self):
-        """0 (1 would be a bounded wait in a kernel that gave up)."""
+        """0, or 1 if a bounded wait in the tensor-core kernel gave up."""
         st = C.c_int()
         check(lib().gbfem_preconditioner_status(self.handle, C.byref(st)))
         return st.value

@@ -50,6 +50,14 @@ RESULTS = {
                  '0x1.5b3882d92c508p-14', '0x1.137754a337aa6p-11', '0x1.5c9e656252120p-12'),
     (4, 'fma'): ('0x1.5530a600e4d65p-18', '0x1.1a135edcfd48fp-14', '0x1.1ebaa6c76530fp-14',
                  '0x1.cd71a4c410e2ep-17', '0x1.794e3e440c769p-14', '0x1.cf3085266557cp-15'),
+    (1, 'tensor'): ('0x1.1cfde259cd703p-10', '0x1.6b5f48101ea50p-6', '0x1.7b22e26f2d962p-6',
+                 '0x1.da7fa6aed70ccp-9', '0x1.ddf9f796fc29bp-6', '0x1.1d91e2032894ep-6'),
+    (2, 'tensor'): ('0x1.bfff2273b1f7fp-13', '0x1.89f9d282c42e1p-9', '0x1.924f712e77133p-9',
+                 '0x1.3c10e398bad45p-11', '0x1.04b9272406b71p-8', '0x1.44fa855d33086p-9'),
+    (3, 'tensor'): ('0x1.de8a3a246218bp-16', '0x1.a1ebeaa51e4b7p-12', '0x1.ab1b95caaa7dbp-12',
+                 '0x1.5b3797e6aeb1ep-14', '0x1.1376ea3cda877p-11', '0x1.5c9d548090448p-12'),
+    (4, 'tensor'): ('0x1.55318d36c9b72p-18', '0x1.1a143ab635676p-14', '0x1.1ebb9de7475a4p-14',
+                 '0x1.cd731c499a874p-17', '0x1.794f779f4e6c1p-14', '0x1.cf31d8375a080p-15'),
 }
 
 
