@@ -390,12 +390,14 @@ __global__ void __launch_bounds__(fx_threads<N, FxBrick<N, SMALL>>(), FxBrick<N,
           if (args.weak_dirichlet) lo = FxPair{-own0.v, (fx.slope ? 0 : own0.v) - own0.p};
         }
         // without diffusion the outflow neighbour has no part in the line, and its
-        // magnitude must not either
+        // magnitude must not either (au, al: the exponents to align at; eu, el stay what
+        // the neighbours' traces are held in)
+        int au = eu, al = el;
         if (ADV) {
-          if (!fx.couple[D][1] && eu != kFxSlow) eu = eo[r];
-          if (!fx.couple[D][0] && el != kFxSlow) el = eo[r];
+          if (!fx.couple[D][1] && eu != kFxSlow) au = eo[r];
+          if (!fx.couple[D][0] && el != kFxSlow) al = eo[r];
         }
-        const int ef = max(eo[r], max(eu, el));
+        const int ef = max(eo[r], max(au, al));
         double* const rc = res + (c0 + r * (B::X * B::Y * B::L)) * N3;
         double y[N];
         if (D == 0) {
@@ -406,7 +408,7 @@ __global__ void __launch_bounds__(fx_threads<N, FxBrick<N, SMALL>>(), FxBrick<N,
           for (int i = 0; i < N; ++i) y[i] = rc[fx_res_off<N, D>(jk, i)];
         }
         if (ef != kFxSlow) {
-          const int so = min(ef - eo[r], 63), su = min(ef - eu, 63), sl = min(ef - el, 63);
+          const int so = min(ef - eo[r], 63), su = min(ef - au, 63), sl = min(ef - al, 63);
           const long long vu = fx_shr(up.v, su), vl = fx_shr(lo.v, sl);
           const long long J1 = fx_shr(own1.v, so) - vu, P1 = fx_shr(own1.p, so) - fx_shr(up.p, su);
           const long long J0 = fx_shr(own0.v, so) - vl, P0 = fx_shr(own0.p, so) - fx_shr(lo.p, sl);

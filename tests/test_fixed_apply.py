@@ -198,3 +198,22 @@ def test_refused_coefficients_take_the_fp64_kernels(gb):
     cells, u = (5, 4, 3), np.random.default_rng(3).uniform(-1.0, 1.0, 5 * 4 * 3 * 64)
     w, w2 = apply_both(gb, cells, 3, u, penalty=1e-3)
     assert np.max(np.abs(w - w2)) <= 1e-12 * np.max(np.abs(w2))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("velocity", [(1.0, -0.5, 0.25), (1.0, 0.0, 0.0)])
+def test_extreme_lines_beside_uncoupled_neighbours(gb, order, velocity):
+    """Without diffusion an outflow neighbour, or any neighbour along an axis
+    without velocity, has no part in a line: lines that fixed point cannot hold
+    beside ordinary ones, each within 2^-48 of its own terms."""
+    kw, cells = dict(diffusion=0.0, velocity=velocity), (5, 4, 6)
+    n3 = (order + 1) ** 3
+    base = np.random.default_rng(order).uniform(-1.0, 1.0, (np.prod(cells), n3))
+    for mark in (1e-250, 1e-300, 1e280):
+        u = base.copy()
+        u[[7, 60, 61, 93]] *= mark
+        u = u.ravel()
+        w = apply_both(gb, cells, order, u, **kw)[0]
+        ref, size = reference(cells, order, u, **kw)
+        assert np.all(np.abs(w - ref) <= 2.0 ** -48 * size + 64 * 5e-324), mark
