@@ -29,7 +29,15 @@ struct FxBasis {
 // The tables of a constant-kappa operator, from the descriptor in long double
 // and rounded once; false where its coefficients do not fit the fixed-point
 // ranges (a penalty so small that the trace P = v - r dv outgrows v, scales
-// beyond 2^+-kFxRowExpMax).
+// beyond 2^+-kFxRowExpMax) or where a line would hold fewer bits than in FP64: a row
+// is formed at the largest exponent of its line and its neighbours', so every line that
+// takes part has to weigh in it.  With V = sum L_j(1), a penalty alone weighs between
+// V / 64 and V / 32 of the row's scale 2^e (which covers the face's 32 L_i); the least
+// accepted is 0.009 (1 + V).  Error against 128 bits, entry by entry over all ratios of
+// the neighbours' sizes, root mean square relative to FP64's: above that line 0.3-1.3
+// (up to 1.6 where a line's own coefficients differ by 2^40, with p = 1; there also
+// 1.4 far above it); below, at velocity 1 and h = 1/8: p = 1 3 (diffusion 1e-3), p = 2 6
+// and 860 (1e-4 and 1e-6).
 bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
   *out = FxTables{};
   if (d.kappa || d.kappa_cell) return false;
@@ -51,7 +59,7 @@ bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
     const long double A2 = area * eps * 0.5L / h[k];
     const long double C = sipg ? area * eps * d.penalty / h[k] : 1.0L, r = A2 / C;
     if (!std::isfinite(double(r)) || !std::isfinite(double(C))) return false;
-    long double cls[2] = {0.0L, 0.0L}, slope = 0.0L;
+    long double cls[2] = {0.0L, 0.0L}, slope = 0.0L, vsum = 0.0L;
     for (int i = 0; i < n; ++i) {
       // without penalty (C = 1) P - v = -r dv is what the flux takes, and it is
       // held as such: P itself would carry it below the digits of v
@@ -63,6 +71,9 @@ bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
       ax.P[i] = fx_coef(p / 8.0L, 62);
     }
     if (!(cls[0] <= kFxClassSum && cls[1] <= kFxClassSum && slope <= 2 * kFxClassSum)) return false;
+    for (int i = 0; i < n; ++i) vsum += fabsl(L[i]);
+    // a line without any face term
+    if (d.grid.cells[k] == 1 && !d.weak_dirichlet && (eps != 0.0L || b != 0.0L || (k == 0 && d.mass != 0.0))) return false;
     // inflow and outflow faces: b.n < 0 and > 0
     const int out_side = b > 0.0L ? 1 : 0, in_side = 1 - out_side;
     out->inflow_upper[k] = in_side;
@@ -86,6 +97,12 @@ bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
       if (!std::isfinite(double(big))) return false;
       if (big > 0.0L) frexpl(big, &e);  // big < 2^e
       if (e > kFxRowExpMax || e < -kFxRowExpMax) return false;
+      for (int side = 0; side < 2 && big > 0.0L; ++side) {
+        const long double w = fabsl(np) * (cls[0] + cls[1]) + (fabsl(nv) + (side == in_side ? fabsl(a) : 0.0L)) * vsum;
+        if (out->couple[k][side] && !(w >= 32.0L * 0.009L * (1.0L + vsum) * ldexpl(1.0L, e))) return false;
+      }
+      // nothing but the mass: an entry has no part in the others of its line
+      if (big > 0.0L && !out->couple[k][0] && !out->couple[k][1]) return false;
       for (int j = 0; j < n; ++j) ax.O[i * n + j] = fx_coef(ldexpl(O[j], -e), bits);
       ax.np[i] = fx_coef(ldexpl(np, -e), bits);
       ax.nv[i] = fx_coef(ldexpl(nv, -e), bits);

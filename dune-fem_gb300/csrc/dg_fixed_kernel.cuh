@@ -26,8 +26,9 @@
 //
 // Exponents: each line has its own (its largest coefficient), its traces carry
 // it, and the line's result is formed at the largest of its own and its two
-// neighbours'.  So an entry is as exact relative to the line it belongs to as
-// an FP64 sum is, whatever the rest of the cell holds: one unit of a trace is
+// neighbours', the lines that enter it with weight (fx_make_tables refuses the
+// operators where one hardly does).  So an entry is as exact relative to these lines
+// as an FP64 sum is, whatever the rest of the cell holds: one unit of a trace is
 // 2^-56 of the line's binade, where an FP64 trace rounds at 2^-53 of its value.
 // Lines that fixed point cannot hold (infinities, NaN, magnitudes outside
 // 2^-822 .. 2^777) are computed by the FP64 formulas instead, line by line.
