@@ -41,6 +41,10 @@ struct FxBasis {
 bool fx_make_tables(const gbfem_dg_desc& d, int n, FxTables* out) {
   *out = FxTables{};
   if (d.kappa || d.kappa_cell) return false;
+  // (a NaN would be lost in the integers; fmaxl drops it too)
+  if (!std::isfinite(d.mass) || !std::isfinite(d.velocity[0]) || !std::isfinite(d.velocity[1]) ||
+      !std::isfinite(d.velocity[2]))
+    return false;
   static const FxBasis bases[4] = {FxBasis(2), FxBasis(3), FxBasis(4), FxBasis(5)};
   const ConstTables1D& ct = bases[n - 2].ct;
   const long double *L = bases[n - 2].L, *dL = bases[n - 2].dL;

@@ -217,3 +217,14 @@ def test_extreme_lines_beside_uncoupled_neighbours(gb, order, velocity):
         w = apply_both(gb, cells, order, u, **kw)[0]
         ref, size = reference(cells, order, u, **kw)
         assert np.all(np.abs(w - ref) <= 2.0 ** -48 * size + 64 * 5e-324), mark
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [dict(mass=np.nan), dict(velocity=(0.5, np.nan, 0.0)), dict(velocity=(0.5, np.inf, 0.0)),
+                                dict(diffusion=np.nan), dict(penalty=np.nan)])
+def test_non_finite_coefficients(gb, kw):
+    """The result is not finite either."""
+    op = gb.DGOperator((3, 4, 2), 2, **kw)
+    w = gb.DeviceArray(op.size)
+    op(gb.DeviceArray.from_numpy(np.random.default_rng(1).uniform(0.5, 1.0, op.size)), w)
+    assert not np.any(np.isfinite(w.numpy().reshape(-1, 27)[:, 0]))
