@@ -21,13 +21,14 @@
 // warp of every CTA polls all parts and adds them in the same order.  All CTAs
 // so take the same decisions on the same bits.  Two sets of slots alternate: a
 // CTA that writes sum k+2 has seen every part of sum k+1, hence every CTA is done
-// reading sum k.  The polls are bounded; a CTA that gives up reports it and
-// leaves.  The statements are those of LinearSolver::cg (solver/linear/cg.hh:
+// reading sum k.  The polls of a wait are bounded; a CTA that gives up sets a word that
+// the host checks and leaves.  The statements are those of LinearSolver::cg (solver/linear/cg.hh:
 // 18-117) on p = b - A x; without a preconditioner s = p.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <climits>
 #include <cmath>
+#include <cstring>
 
 #include "blas.cuh"
 #include "gbfem_internal.cuh"
@@ -40,7 +41,7 @@ constexpr int kQ1Threads = 256;
 constexpr int kQ1MaxPer = 8;           // vertices per thread
 constexpr int kQ1MaxCluster = 16;
 constexpr int kQ1MaxGrid = 160;        // CTAs (one per SM)
-constexpr int kQ1PollLimit = 1 << 20;  // polls of a grid-wide sum (about a second)
+constexpr int kQ1PollLimit = 1 << 20;  // polls of one wait, a sum or a halo (about a second)
 
 struct Q1CgArgs {
   const void *b, *dinv;
@@ -48,6 +49,8 @@ struct Q1CgArgs {
   unsigned long long* slots;  // [2][grid][2]: tagged parts of the grid-wide sums
   unsigned long long* s;      // [n][2]: tagged s, for the neighbours' halos
   double* out;                // residual, iterations, status, tolerance, beta
+  int* late;                  // set by a CTA that gave up
+  int late_cta;               // this CTA's waits all run out (self test; -1: none)
   int resume;
   int n, vxn, vyn, per_cta;
   double c[9];                // stencil, row by row from the lower left vertex
@@ -83,13 +86,13 @@ __device__ __forceinline__ void q1_put(unsigned long long* at, double v, unsigne
   w[0] = t | (bits & 0xffffffffull);
   w[1] = t | (bits >> 32);
 }
-__device__ __forceinline__ double q1_get(const unsigned long long* at, unsigned tag, int& polls) {
+__device__ __forceinline__ double q1_get(const unsigned long long* at, unsigned tag, int limit, int& polls) {
   const volatile unsigned long long* w = at;
   unsigned long long a = 0, b = 0;
   do {
     a = w[0];
     b = w[1];
-  } while (((unsigned)(a >> 32) != tag || (unsigned)(b >> 32) != tag) && ++polls < kQ1PollLimit);
+  } while (((unsigned)(a >> 32) != tag || (unsigned)(b >> 32) != tag) && ++polls < limit);
   return __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
 }
 
@@ -101,10 +104,9 @@ __device__ __forceinline__ double q1_get(const unsigned long long* at, unsigned 
 // comes out of a divergent loop.)
 template <bool CLUSTER>
 __device__ __forceinline__ bool q1_grid_sum(double v, double other, bool inverse, unsigned epoch,
-                                            unsigned long long* slots, Q1Shared& sh, int polls) {
+                                            unsigned long long* slots, Q1Shared& sh, int limit) {
   const int tid = threadIdx.x, grid = gridDim.x;
   sh.part[tid] = v;
-  if (!CLUSTER && polls >= kQ1PollLimit) sh.late = 1;
   __syncthreads();
   double t = 0.0;
   if (tid < 32) {
@@ -137,10 +139,11 @@ __device__ __forceinline__ bool q1_grid_sum(double v, double other, bool inverse
       unsigned long long* set = slots + (size_t)(epoch & 1u) * grid * 2;
       if (tid == 0) q1_put(set + 2 * blockIdx.x, t, epoch);
       t = 0.0;
-      for (int c = tid; c < grid; c += 32) t += q1_get(set + 2 * c, epoch, polls);
+      int polls = 0;
+      for (int c = tid; c < grid; c += 32) t += q1_get(set + 2 * c, epoch, limit, polls);
       __syncwarp();
       t = q1_warp_sum(t);
-      const bool late = __any_sync(0xffffffffu, polls >= kQ1PollLimit) || sh.late;
+      const bool late = __any_sync(0xffffffffu, polls >= limit) || sh.late;
       const double q = inverse ? t / other : other / t;
       if (tid == 0) {
         sh.sum = t;
@@ -195,10 +198,10 @@ __global__ void __launch_bounds__(kQ1Threads) q1_cg_kernel(const __grid_constant
   if (tid == 0) sh.late = 0;
   if constexpr (CLUSTER) cooperative_groups::this_cluster().sync();  // every CTA runs before its memory is written
   unsigned epoch = 0, tag = 0;
-  int polls = 0;
+  const int limit = int(blockIdx.x) == g.late_cta ? 0 : kQ1PollLimit;
   auto total = [&](double v, double other, bool inverse) {
     ++epoch;
-    return q1_grid_sum<CLUSTER>(v, other, inverse, epoch, g.slots, sh, polls);
+    return q1_grid_sum<CLUSTER>(v, other, inverse, epoch, g.slots, sh, limit);
   };
 
   // p = b - A x, s = P p, q = s (or the state the last launch left)
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(kQ1Threads) q1_cg_kernel(const __grid_constant
   for (; status == Q1_OK && residual > tolerance && it < last; ++it) {
     const T bt = beta;
     each([&](int k, int v) { sq[v - h0] = it > 0 ? s[k] + bt * sq[v - h0] : s[k]; });
+    int polls = 0;
     for (int j = tid; j < (v0 - h0) + (h1 - v1); j += kQ1Threads) {
       const int v = j < v0 - h0 ? h0 + j : v1 + (j - (v0 - h0));
       T sv;
@@ -254,10 +258,11 @@ __global__ void __launch_bounds__(kQ1Threads) q1_cg_kernel(const __grid_constant
         const int c = v / g.per_cta;
         sv = cooperative_groups::this_cluster().map_shared_rank(ss, unsigned(c))[v - c * g.per_cta];
       } else {
-        sv = T(q1_get(g.s + 2ll * v, tag, polls));
+        sv = T(q1_get(g.s + 2ll * v, tag, limit, polls));
       }
       sq[v - h0] = it > 0 ? sv + bt * sq[v - h0] : sv;
     }
+    if (!CLUSTER && polls >= limit) sh.late = 1;
     __syncthreads();
     DotAcc<T> qh;
     each([&](int k, int v) {
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(kQ1Threads) q1_cg_kernel(const __grid_constant
       pg[v] = p[k];
       qg[v] = sq[v - h0];
     });
+  if (status == Q1_TIMEOUT && tid == 0) atomicExch(g.late, 1);
   if (blockIdx.x == 0 && tid == 0) {
     g.out[Q1_RES] = residual;
     g.out[Q1_IT] = double(it);
@@ -356,7 +362,7 @@ bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_
 }
 
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
-          cudaStream_t s, gbfem_solver_info* info) {
+          cudaStream_t s, gbfem_solver_info* info, const Q1Trial* trial) {
   int dev = 0, sms = 0;
   GBFEM_CUDA_TRY(cudaGetDevice(&dev));
   GBFEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -369,7 +375,7 @@ int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params&
   // through distributed shared memory (65^2: 5.0 us an iteration, 7.2 with the
   // sums through L2); beyond, where 16 SMs' FP64 work outweighs that, the whole GPU
   // (121^2: 8.4 us with one cluster; 151^2: 11.1 us over 90 SMs).
-  const bool cluster = a.n <= kQ1MaxCluster * 1024;
+  const bool cluster = a.n <= kQ1MaxCluster * 1024 && !(trial && trial->no_cluster);
   int grid = (a.n + kQ1Threads - 1) / kQ1Threads;
   if (cluster) {
     const int want = (a.n + 63) / 64;
@@ -390,19 +396,23 @@ int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params&
   a.b = b;
   a.x = x;
   a.dinv = pc ? pc->data : nullptr;
+  a.late_cta = trial ? trial->late_cta : -1;
   const size_t es = op->precision == GBFEM_F64 ? 8 : 4;
   const size_t vec = (size_t(a.n) * es + 15) / 16 * 16, slots = size_t(2) * grid * 16 + size_t(a.n) * 16;
   struct Buffer {
     char* p = nullptr;
     ~Buffer() { if (p) cudaFree(p); }
   } buf;
-  GBFEM_CUDA_TRY(cudaMalloc(&buf.p, 2 * vec + slots + Q1_OUT * sizeof(double)));
+  constexpr int kOut = Q1_OUT + 1;  // out, and the late word in a double's place
+  GBFEM_CUDA_TRY(cudaMalloc(&buf.p, 2 * vec + slots + kOut * sizeof(double)));
   a.p = buf.p;
   a.q = buf.p + vec;
   a.slots = reinterpret_cast<unsigned long long*>(buf.p + 2 * vec);
   a.s = a.slots + size_t(4) * grid;
   a.out = reinterpret_cast<double*>(buf.p + 2 * vec + slots);
-  double out[Q1_OUT];
+  a.late = reinterpret_cast<int*>(a.out + Q1_OUT);
+  double out[kOut];
+  GBFEM_CUDA_TRY(cudaMemsetAsync(a.late, 0, sizeof(double), s));
   for (;;) {
     GBFEM_CUDA_TRY(cudaMemsetAsync(a.slots, 0, slots, s));
     const cudaError_t e =
@@ -411,7 +421,9 @@ int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params&
     if (e != cudaSuccess) return set_cuda_error(e, "q1 cg");
     GBFEM_CUDA_TRY(cudaMemcpyAsync(out, a.out, sizeof(out), cudaMemcpyDeviceToHost, s));
     GBFEM_CUDA_TRY(cudaStreamSynchronize(s));
-    if (int(out[Q1_STATUS]) == Q1_TIMEOUT) return set_error(GBFEM_ERR_CUDA, "q1 cg: a grid-wide sum did not complete");
+    int late;
+    std::memcpy(&late, out + Q1_OUT, sizeof(late));
+    if (late) return set_error(GBFEM_ERR_CUDA, "q1 cg: a grid-wide sum did not complete");
     if (int(out[Q1_STATUS]) != Q1_OK || !(out[Q1_RES] > out[Q1_TOL]) || int(out[Q1_IT]) >= a.max_it) break;
     a.resume = 1;
   }

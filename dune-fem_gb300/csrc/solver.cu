@@ -1547,6 +1547,15 @@ int gbfem_solve(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_p
   return solve_impl(op, pc, *prm, f, u, info, nullptr, nullptr);
 }
 
+int gbfem_selftest_q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params* prm, const void* f,
+                         void* u, gbfem_solver_info* info, int late_cta, int no_cluster) {
+  if (!op || !prm || !f || !u || !info) return set_error(GBFEM_ERR_INVALID, "gbfem_selftest_q1_cg: null argument");
+  if (!q1_cg_takes(op, pc, *prm)) return set_error(GBFEM_ERR_INVALID, "gbfem_selftest_q1_cg: not a solve of that kernel");
+  *info = gbfem_solver_info{};
+  const Q1Trial trial{late_cta, no_cluster};
+  return q1_cg(op, pc, *prm, f, u, nullptr, info, &trial);
+}
+
 }  // extern "C"
 
 namespace gbfem {

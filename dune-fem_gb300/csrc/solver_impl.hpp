@@ -29,9 +29,13 @@ int cg_apply_dot(const struct ::gbfem_operator_s* op, const void* q, void* h, do
                  cudaStream_t s);
 int dg_mixed_form(struct ::gbfem_operator_s* op, struct ::gbfem_operator_s* keep, struct ::gbfem_operator_s** out);
 // the Q1 operator's CG in one kernel (q1_cg.cu), for the solves it takes
+struct Q1Trial {     // self test
+  int late_cta;      // a CTA whose waits all run out, -1: none
+  int no_cluster;    // as if no cluster could be placed
+};
 bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
-          cudaStream_t s, gbfem_solver_info* info);
+          cudaStream_t s, gbfem_solver_info* info, const Q1Trial* trial = nullptr);
 
 }  // namespace gbfem
 

@@ -1,5 +1,7 @@
 """The one-kernel CG of the Q1 operator against the oracle's CG on the oracle's
 operator, over grids of one CTA, ragged ranges, and several vertices a thread."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -85,4 +87,35 @@ def test_start_vector_precision_and_stops(gb):
     inv(fd, u)
     info = inv.info()
     assert info["iterations"] == -20000 or info["residual"] == 0.0 or info["status"] != 0
+    assert np.max(np.abs(u.numpy() - ref)) <= 1e-9 * np.max(np.abs(ref))
+
+
+def _selftest(gb, op, pc, f, u, late_cta, no_cluster, **kw):
+    prm, info = gb.solver_params("cg", 1e-12, **kw), gb.SolverInfo()
+    rc = gb.lib().gbfem_selftest_q1_cg(op.handle, pc.handle, C.byref(prm), f.ptr, u.ptr, C.byref(info),
+                                       C.c_int(late_cta), C.c_int(no_cluster))
+    return rc, info
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("late_cta", [0, 3, 5])
+@pytest.mark.parametrize("iterations", [0, 50])
+def test_a_block_that_gives_up_is_an_error(gb, late_cta, iterations):
+    """Whichever block it is and whenever: without iterations the other blocks get
+    all parts of the only sum and end as if all were well.  The next solve is
+    unaffected."""
+    cells = (40, 33)  # 1394 vertices, 6 blocks
+    f, ref = _rhs(cells, 7), _exact(cells, _rhs(cells, 7))
+    op = gb.Q1Operator(cells, diffusion=1.0, mass=1.0)
+    pc = gb.Preconditioner.diagonal(op)
+    fd, u = gb.DeviceArray.from_numpy(f), gb.DeviceArray(op.size)
+    u.clear()
+    kw = dict(error_measure=gb.ABSOLUTE, max_iterations=iterations)
+    rc, _ = _selftest(gb, op, pc, fd, u, late_cta, 1, **kw)
+    assert rc != 0
+    u.clear()
+    assert _selftest(gb, op, pc, fd, u, -1, 1, **kw)[0] == 0
+    u.clear()
+    rc, info = _selftest(gb, op, pc, fd, u, -1, 1)
+    assert rc == 0 and info.converged
     assert np.max(np.abs(u.numpy() - ref)) <= 1e-9 * np.max(np.abs(ref))
