@@ -307,8 +307,9 @@ __global__ void __launch_bounds__(kQ1Threads) q1_cg_kernel(const __grid_constant
   }
 }
 
+// fits: ask only whether the device can hold the launch
 template <typename T, int PER>
-static cudaError_t q1_launch(const Q1CgArgs& a, int grid, bool cluster, cudaStream_t s) {
+static cudaError_t q1_launch(const Q1CgArgs& a, int grid, bool cluster, cudaStream_t s, bool* fits) {
   const size_t smem = size_t(2 * a.per_cta + 2 * (a.vxn + 1)) * sizeof(T);
   auto kern = cluster ? q1_cg_kernel<T, PER, true> : q1_cg_kernel<T, PER, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -331,16 +332,33 @@ static cudaError_t q1_launch(const Q1CgArgs& a, int grid, bool cluster, cudaStre
   }
   cfg.attrs = &at;
   cfg.numAttrs = 1;
+  if (fits) {
+    int dev = 0, sms = 0, held = 0;
+    if (cluster) {
+      e = cudaOccupancyMaxActiveClusters(&held, kern, &cfg);
+      *fits = e == cudaSuccess && held > 0;
+    } else {
+      e = cudaGetDevice(&dev);
+      if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&held, kern, kQ1Threads, smem);
+      *fits = e == cudaSuccess && (long long)held * sms >= grid;
+    }
+    return e;
+  }
   return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
 template <typename T>
-static cudaError_t q1_launch_per(const Q1CgArgs& a, int grid, bool cluster, cudaStream_t s) {
+static cudaError_t q1_launch_per(const Q1CgArgs& a, int grid, bool cluster, cudaStream_t s, bool* fits) {
   const int per = (a.per_cta + kQ1Threads - 1) / kQ1Threads;
-  if (per <= 1) return q1_launch<T, 1>(a, grid, cluster, s);
-  if (per <= 2) return q1_launch<T, 2>(a, grid, cluster, s);
-  if (per <= 4) return q1_launch<T, 4>(a, grid, cluster, s);
-  return q1_launch<T, kQ1MaxPer>(a, grid, cluster, s);
+  if (per <= 1) return q1_launch<T, 1>(a, grid, cluster, s, fits);
+  if (per <= 2) return q1_launch<T, 2>(a, grid, cluster, s, fits);
+  if (per <= 4) return q1_launch<T, 4>(a, grid, cluster, s, fits);
+  return q1_launch<T, kQ1MaxPer>(a, grid, cluster, s, fits);
+}
+static cudaError_t q1_launch_any(int precision, const Q1CgArgs& a, int grid, bool cluster, cudaStream_t s, bool* fits) {
+  return precision == GBFEM_F64 ? q1_launch_per<double>(a, grid, cluster, s, fits)
+                                : q1_launch_per<float>(a, grid, cluster, s, fits);
 }
 
 // Whether q1_cg takes the solve: no per-iteration output, the stops of the CG
@@ -361,8 +379,9 @@ bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_
          (2LL * kQ1Threads * kQ1MaxPer + halo) * 8 <= 200 * 1024;
 }
 
+// *taken false: nothing is done, the device cannot hold the kernel.
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
-          cudaStream_t s, gbfem_solver_info* info, const Q1Trial* trial) {
+          cudaStream_t s, gbfem_solver_info* info, bool* taken, const Q1Trial* trial) {
   int dev = 0, sms = 0;
   GBFEM_CUDA_TRY(cudaGetDevice(&dev));
   GBFEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -374,16 +393,28 @@ int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params&
   // Up to 16384 vertices: one cluster of at most 16 CTAs, whose sums and halos go
   // through distributed shared memory (65^2: 5.0 us an iteration, 7.2 with the
   // sums through L2); beyond, where 16 SMs' FP64 work outweighs that, the whole GPU
-  // (121^2: 8.4 us with one cluster; 151^2: 11.1 us over 90 SMs).
-  const bool cluster = a.n <= kQ1MaxCluster * 1024 && !(trial && trial->no_cluster);
-  int grid = (a.n + kQ1Threads - 1) / kQ1Threads;
-  if (cluster) {
-    const int want = (a.n + 63) / 64;
-    for (grid = 1; grid < want && grid < kQ1MaxCluster;) grid *= 2;
+  // (121^2: 8.4 us with one cluster; 151^2: 11.1 us over 90 SMs), and where the device
+  // cannot place such a cluster; the general loop where it can hold neither.
+  bool cluster = a.n <= kQ1MaxCluster * 1024, fits = false;
+  int grid = 0;
+  for (;; cluster = false) {
+    grid = (a.n + kQ1Threads - 1) / kQ1Threads;
+    if (cluster) {
+      const int want = (a.n + 63) / 64;
+      for (grid = 1; grid < want && grid < kQ1MaxCluster;) grid *= 2;
+    }
+    if (grid > sms) grid = sms;
+    a.per_cta = (a.n + grid - 1) / grid;
+    if (!cluster) grid = (a.n + a.per_cta - 1) / a.per_cta;  // (a cluster's last CTAs may be empty)
+    if (q1_launch_any(op->precision, a, grid, cluster, s, &fits) != cudaSuccess) {
+      (void)cudaGetLastError();
+      fits = false;
+    }
+    if (trial && (cluster ? trial->no_cluster : trial->no_grid)) fits = false;
+    if (fits || !cluster) break;
   }
-  if (grid > sms) grid = sms;
-  a.per_cta = (a.n + grid - 1) / grid;
-  if (!cluster) grid = (a.n + a.per_cta - 1) / a.per_cta;  // (a cluster's last CTAs may be empty)
+  *taken = fits;
+  if (!fits) return GBFEM_OK;
   // the four elements around a vertex: element (cx, cy) has it as its corner
   // (1 - cx) + 2 (1 - cy)
   for (int cy = 0; cy < 2; ++cy)
@@ -415,9 +446,7 @@ int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params&
   GBFEM_CUDA_TRY(cudaMemsetAsync(a.late, 0, sizeof(double), s));
   for (;;) {
     GBFEM_CUDA_TRY(cudaMemsetAsync(a.slots, 0, slots, s));
-    const cudaError_t e =
-        op->precision == GBFEM_F64 ? q1_launch_per<double>(a, grid, cluster, s)
-                                     : q1_launch_per<float>(a, grid, cluster, s);
+    const cudaError_t e = q1_launch_any(op->precision, a, grid, cluster, s, nullptr);
     if (e != cudaSuccess) return set_cuda_error(e, "q1 cg");
     GBFEM_CUDA_TRY(cudaMemcpyAsync(out, a.out, sizeof(out), cudaMemcpyDeviceToHost, s));
     GBFEM_CUDA_TRY(cudaStreamSynchronize(s));

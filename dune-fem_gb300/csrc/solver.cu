@@ -1212,16 +1212,17 @@ static int fcg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_pa
 }
 
 int solve_impl(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* f, void* u,
-               gbfem_solver_info* info, cudaStream_t s, CgDeviceState* keep) {
+               gbfem_solver_info* info, cudaStream_t s, CgDeviceState* keep, const Q1Trial* trial = nullptr) {
   *info = gbfem_solver_info{};
   const auto t0 = std::chrono::steady_clock::now();
   int rc;
   if (prm.error_measure < GBFEM_TOL_ABSOLUTE || prm.error_measure > GBFEM_TOL_RELATIVE_RESIDUAL)
     return set_error(GBFEM_ERR_INVALID, "gbfem_solve: unknown error measure");
   if (prm.method == GBFEM_SOLVER_CG && q1_cg_takes(op, pc, prm)) {
-    rc = q1_cg(op, pc, prm, f, u, s, info);
+    bool taken = false;
+    rc = q1_cg(op, pc, prm, f, u, s, info, &taken, trial);
     info->time_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    return rc;
+    if (rc || taken) return rc;
   }
   Ctx c;
   GBFEM_TRY(c.setup(op->precision, op->ndofs, s));
@@ -1548,12 +1549,11 @@ int gbfem_solve(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_p
 }
 
 int gbfem_selftest_q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params* prm, const void* f,
-                         void* u, gbfem_solver_info* info, int late_cta, int no_cluster) {
+                         void* u, gbfem_solver_info* info, int late_cta, int no_cluster, int no_grid) {
   if (!op || !prm || !f || !u || !info) return set_error(GBFEM_ERR_INVALID, "gbfem_selftest_q1_cg: null argument");
   if (!q1_cg_takes(op, pc, *prm)) return set_error(GBFEM_ERR_INVALID, "gbfem_selftest_q1_cg: not a solve of that kernel");
-  *info = gbfem_solver_info{};
-  const Q1Trial trial{late_cta, no_cluster};
-  return q1_cg(op, pc, *prm, f, u, nullptr, info, &trial);
+  const Q1Trial trial{late_cta, no_cluster, no_grid};
+  return solve_impl(op, pc, *prm, f, u, info, nullptr, nullptr, &trial);
 }
 
 }  // extern "C"

@@ -32,10 +32,11 @@ int dg_mixed_form(struct ::gbfem_operator_s* op, struct ::gbfem_operator_s* keep
 struct Q1Trial {     // self test
   int late_cta;      // a CTA whose waits all run out, -1: none
   int no_cluster;    // as if no cluster could be placed
+  int no_grid;       // as if the device held fewer blocks than the other form has
 };
 bool q1_cg_takes(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm);
 int q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params& prm, const void* b, void* x,
-          cudaStream_t s, gbfem_solver_info* info, const Q1Trial* trial = nullptr);
+          cudaStream_t s, gbfem_solver_info* info, bool* taken, const Q1Trial* trial);
 
 }  // namespace gbfem
 

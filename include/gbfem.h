@@ -517,11 +517,13 @@ int gbfem_selftest_conversions(uint64_t n, uint64_t seed, uint64_t* mismatches);
 /* y[i] = exp(x[i]) by the integer-arithmetic exp of the FP64 reaction kernels,
  * evaluated on the host (the device runs the same code). */
 int gbfem_selftest_exp(int64_t n, const double* x, double* y);
-/* gbfem_solve of a Q1 operator by the one-kernel CG, where block late_cta (-1:
- * none) gives every wait up at once, and with no_cluster != 0 in the form for
- * grids beyond one cluster.  A block that gave up makes it an error. */
+/* gbfem_solve of a Q1 operator that the one-kernel CG takes, where block late_cta
+ * (-1: none) gives every wait up at once (an error), as if the device could not
+ * place its cluster (no_cluster != 0: the form for larger grids), nor the blocks of
+ * that form (no_grid != 0: the general loop). */
 int gbfem_selftest_q1_cg(gbfem_operator op, gbfem_preconditioner pc, const gbfem_solver_params* params,
-                         const void* f, void* u, gbfem_solver_info* info, int late_cta, int no_cluster);
+                         const void* f, void* u, gbfem_solver_info* info, int late_cta, int no_cluster,
+                         int no_grid);
 int gbfem_cnn_set_output_scale(gbfem_cnn cnn, double scale);
 int gbfem_cnn_get_output_scale(gbfem_cnn cnn, double* scale);
 /* z = S rms(r) NN(r/rms(r)) (accumulate = 1: z += ...). */

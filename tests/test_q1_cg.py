@@ -90,10 +90,10 @@ def test_start_vector_precision_and_stops(gb):
     assert np.max(np.abs(u.numpy() - ref)) <= 1e-9 * np.max(np.abs(ref))
 
 
-def _selftest(gb, op, pc, f, u, late_cta, no_cluster, **kw):
+def _selftest(gb, op, pc, f, u, late_cta, no_cluster, no_grid=0, **kw):
     prm, info = gb.solver_params("cg", 1e-12, **kw), gb.SolverInfo()
     rc = gb.lib().gbfem_selftest_q1_cg(op.handle, pc.handle, C.byref(prm), f.ptr, u.ptr, C.byref(info),
-                                       C.c_int(late_cta), C.c_int(no_cluster))
+                                       C.c_int(late_cta), C.c_int(no_cluster), C.c_int(no_grid))
     return rc, info
 
 
@@ -119,3 +119,22 @@ def test_a_block_that_gives_up_is_an_error(gb, late_cta, iterations):
     rc, info = _selftest(gb, op, pc, fd, u, -1, 1)
     assert rc == 0 and info.converged
     assert np.max(np.abs(u.numpy() - ref)) <= 1e-9 * np.max(np.abs(ref))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cells", [(1, 1), (7, 3), (64, 64)])
+@pytest.mark.parametrize("no_cluster,no_grid", [(0, 0), (1, 0), (1, 1)])
+def test_where_the_device_cannot_place_it(gb, cells, no_cluster, no_grid):
+    """Without room for a cluster the other form, without room for that the general
+    loop: the same solution, and as many iterations within 2 %."""
+    f, ref = _rhs(cells, 3), _exact(cells, _rhs(cells, 3))
+    op = gb.Q1Operator(cells, diffusion=1.0, mass=1.0)
+    pc = gb.Preconditioner.diagonal(op)
+    fd, u, its = gb.DeviceArray.from_numpy(f), gb.DeviceArray(op.size), []
+    for forms in ((0, 0), (no_cluster, no_grid)):
+        u.clear()
+        rc, info = _selftest(gb, op, pc, fd, u, -1, *forms)
+        assert rc == 0 and info.converged
+        assert np.max(np.abs(u.numpy() - ref)) <= 1e-9 * max(np.max(np.abs(ref)), 1e-300)
+        its.append(info.iterations)
+    assert abs(its[0] - its[1]) <= max(2, its[0] // 50)
