@@ -67,7 +67,7 @@ bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out) {
   }
   if (!std::isfinite(double(sum)) || !(sum > 0.0L)) return false;
   out->lDt = qx_scale(big, sum, 2.5L);
-  if (out->lDt > kFxRowExpMax || out->lDt < -kFxRowExpMax) return false;
+  if (out->lDt > kFxRowExpMax || out->lDt < kQxRowExpMin) return false;
   for (int k = 0; k < 3; ++k)
     for (int o = 0; o < q; ++o)
       for (int a = 0; a < q; ++a) out->Dt[k][o * q + a] = qx_coef(Dt[k][o][a], out->lDt);
@@ -91,7 +91,7 @@ bool qx_make_tables(const gbfem_dg_desc& d, int n, int q, QxTables* out) {
       const long double a = cv * t.tr[1][i], b = cg * t.dtr[1][i];
       if (!std::isfinite(double(a)) || !std::isfinite(double(b))) return false;
       const int e = qx_scale(fmaxl(fabsl(a), fabsl(b)), fabsl(a) + fabsl(b), 2.0L);
-      if (e > kFxRowExpMax || e < -kFxRowExpMax) return false;
+      if (e > kFxRowExpMax || e < kQxRowExpMin) return false;
       out->lF[k][i] = e;
       out->fv[k][i] = qx_coef(a, e);
       out->fg[k][i] = qx_coef(b, e);

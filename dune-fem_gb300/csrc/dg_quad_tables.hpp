@@ -11,6 +11,11 @@ namespace gbfem {
 constexpr int kQxMinExp = 400, kQxMaxExp = 1600;  // biased exponents of u
 constexpr int kQxKappaSpan = 100;                 // kappa within 2^+-100
 constexpr int kQxSlow = 0xFFFF;
+// smallest log2 of a scale of the operator.  A result's scale 2^x, built as an exponent
+// field, is smallest where a cell and its neighbours are zero: x = 400 - 1022 (u), - 209
+// (47 bits of the contractions, 6 27 shifts of zero magnitudes), - 99 (kappa) and this:
+// at -93 the field is 1.
+constexpr int kQxRowExpMin = -90;
 
 struct QxTables {
   FxCoef B[kDgMaxQ * kDgMaxN];        // B[a n + i], S = 2^lB

@@ -151,3 +151,19 @@ def test_values_beyond_the_fixed_point_range(gb, order):
     u, k = fields(cells, order, order, False)
     w, _ = apply_both(gb, cells, order, 0, 0 * u, k)
     assert not w.any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_zero_at_the_ends_of_the_scales(gb, order):
+    """u = 0 gives 0 where operator and kappa are as small as fixed point takes them."""
+    cells, n3 = (2, 2, 3), (order + 1) ** 3
+    k = np.zeros((12, n3))
+    u, w = gb.DeviceArray(12 * n3), gb.DeviceArray(12 * n3)
+    u.clear()
+    for e in range(80, 101):
+        k[:, 0] = 2.0 ** -e
+        for eps in (2.0 ** -100, 2.0 ** -102, 2.0 ** -104, 2.0 ** -106, 2.0 ** -108):
+            op = gb.DGOperator(cells, order, kappa=gb.DeviceArray.from_numpy(k.ravel()), diffusion=eps)
+            op(u, w)
+            assert not w.numpy().any(), (e, eps)
