@@ -121,13 +121,28 @@ __global__ void qx_kappa_kernel(const double* __restrict__ kq, const double* __r
   }
 }
 
-// kappa's fixed-point values from the operator's FP64 point caches
+static thread_local bool qx_no_memory = false;  // self test
+
+// kappa's fixed-point values from the operator's FP64 point caches.  They take as much
+// memory as those (Q3 2.2 KB per cell, Q4 3.5); where there is none left for them the
+// operator stays on the FP64 kernel, which needs the FP64 values only.
 int qx_kappa(gbfem_operator_s* op) {
   const int q2 = op->q * op->q, q3 = q2 * op->q;
   if (!op->kq_fixed) {
-    GBFEM_CUDA_TRY(cudaMalloc(&op->kq_fixed, size_t(op->ncells) * q3 * 8));
-    GBFEM_CUDA_TRY(cudaMalloc(&op->kf_fixed, size_t(op->ncells) * 6 * q2 * 8));
-    GBFEM_CUDA_TRY(cudaMalloc(&op->ke_fixed, size_t(op->ncells) * 2));
+    void* t[3] = {nullptr, nullptr, nullptr};
+    const size_t bytes[3] = {size_t(op->ncells) * q3 * 8, size_t(op->ncells) * 6 * q2 * 8, size_t(op->ncells) * 2};
+    bool ok = !qx_no_memory;
+    for (int i = 0; i < 3 && ok; ++i) ok = cudaMalloc(&t[i], bytes[i]) == cudaSuccess;
+    if (!ok) {
+      (void)cudaGetLastError();
+      for (void* p : t)
+        if (p) cudaFree(p);
+      op->quad_fixed = false;
+      return GBFEM_OK;
+    }
+    op->kq_fixed = t[0];
+    op->kf_fixed = t[1];
+    op->ke_fixed = t[2];
   }
   long long blocks = (op->ncells + 7) / 8;
   if (blocks > 152LL * 32) blocks = 152LL * 32;
@@ -176,3 +191,8 @@ int dg_quad_fixed_launch(const gbfem_operator_s* op, const DgArgsT<double>& a, c
 }
 
 }  // namespace gbfem
+
+extern "C" int gbfem_selftest_no_fixed_memory(int on) {
+  gbfem::qx_no_memory = on != 0;
+  return GBFEM_OK;
+}

@@ -517,6 +517,9 @@ int gbfem_selftest_conversions(uint64_t n, uint64_t seed, uint64_t* mismatches);
 /* y[i] = exp(x[i]) by the integer-arithmetic exp of the FP64 reaction kernels,
  * evaluated on the host (the device runs the same code). */
 int gbfem_selftest_exp(int64_t n, const double* x, double* y);
+/* Until called with 0: the operators this thread creates find no memory for the
+ * fixed-point tables of their kappa field. */
+int gbfem_selftest_no_fixed_memory(int on);
 /* gbfem_solve of a Q1 operator that the one-kernel CG takes, where block late_cta
  * (-1: none) gives every wait up at once (an error), as if the device could not
  * place its cluster (no_cluster != 0: the form for larger grids), nor the blocks of

@@ -167,3 +167,28 @@ def test_zero_at_the_ends_of_the_scales(gb, order):
             op = gb.DGOperator(cells, order, kappa=gb.DeviceArray.from_numpy(k.ravel()), diffusion=eps)
             op(u, w)
             assert not w.numpy().any(), (e, eps)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_without_memory_for_the_tables(gb, order):
+    """The operator is made all the same and gives the FP64 kernel's bits, also after
+    an update of kappa."""
+    cells, n3 = (5, 4, 3), (order + 1) ** 3
+    rng = np.random.default_rng(order)
+    k = np.zeros((60, n3))
+    k[:, 0], k[:, 1] = rng.uniform(1.0, 2.0, 60), rng.uniform(-0.2, 0.2, 60)
+    kappa = gb.DeviceArray.from_numpy(k.ravel())
+    u = gb.DeviceArray.from_numpy(rng.uniform(-1.0, 1.0, 60 * n3))
+    ref, w = gb.DeviceArray(60 * n3), gb.DeviceArray(60 * n3)
+    gb.DGOperator(cells, order, kappa=kappa, mass=1e-300)(u, ref)
+    gb.check(gb.lib().gbfem_selftest_no_fixed_memory(1))
+    try:
+        op = gb.DGOperator(cells, order, kappa=kappa)
+    finally:
+        gb.check(gb.lib().gbfem_selftest_no_fixed_memory(0))
+    op(u, w)
+    assert np.array_equal(w.numpy(), ref.numpy())
+    gb.check(gb.lib().gbfem_operator_update_coefficients(op.handle))
+    op(u, w)
+    assert np.array_equal(w.numpy(), ref.numpy())
