@@ -20,7 +20,12 @@
 // coalesced.  Interior cells, in warps that hold nothing else, take V_d from
 // the kernel parameters (uniform operands); other warps read each cell's own
 // from shared memory.  Measured (GB300), tcgen05 3xTF32 tiles of the dense
-// inverse before, this kernel after: 48^3 Q4 94 -> 44 us, 64^3 Q3 116 -> 41.
+// inverse before, this kernel after: 48^3 Q4 94 -> 44 us, 64^3 Q3 116 -> 41; error
+// against 64 bits 9.1e-7 -> 1.4e-7 and 3.8e-7 -> 1.4e-7.
+//
+// For p = 3 and 4 only: with p <= 2 the dense products are FP32 sums of 27 terms at
+// most, error 8e-8 where six rounded contractions have 2.7e-7 (61 x 50 x 58 Q2: 80 us
+// against 16).
 #include <cuda_runtime.h>
 #include <cmath>
 #include <new>
@@ -50,10 +55,10 @@ struct SbFdm {
   static constexpr int N2 = N * N, N3 = N2 * N;
   // cells per CTA (64^3 Q3: 41.3 us with 40 cells, 43.1 with 32, 47.1 with 64; 48^3
   // Q4: 43.6 with 32, 52.7 with 64)
-  static constexpr int CPB = N <= 2 ? 128 : (N == 3 ? 96 : (N == 4 ? 40 : 32));
+  static constexpr int CPB = N == 4 ? 40 : 32;
   static constexpr int T = CPB * N;
   // plane stride in shared memory: 16-byte rows that spread over the banks for
-  // n = 4, odd strides (n = 3, 5) and the 8-bank one of n = 2 as they are
+  // n = 4, the odd stride of n = 5 as it is
   static constexpr int PL = N == 4 ? 20 : N2;
   static constexpr int CS = N * PL;
   static_assert(T % 32 == 0, "whole warps");
@@ -242,13 +247,14 @@ static void sb_eigen(int n, double (&a)[kDgMaxN][kDgMaxN], double (&V)[kDgMaxN][
   }
 }
 
-// The tables, in pc->sb_fdm; left null where a block is singular to FP32 rounding (one
+// The tables, in pc->sb_fdm; left null for p <= 2 (above) and where a block is singular to FP32 rounding (one
 // cell without a boundary term: the division gives infinities, the dense inverse of
 // the rounded block does not).
 int sb_fdm_setup(gbfem_preconditioner_s* pc) {
   const gbfem_operator_s* op = pc->sor_op;
   const gbfem_dg_desc& d = op->dg;
   const int n = op->n;
+  if (n < 4) return GBFEM_OK;
   const ConstTables1D ct = make_const_tables(n);
   auto* t = new (std::nothrow) SbFdmTables{};
   if (!t) return set_error(GBFEM_ERR_INVALID, "out of host memory");
@@ -330,8 +336,6 @@ int sb_fdm_apply(const gbfem_preconditioner_s* pc, const float* r, float* z, cud
   }
   const SbFdmTables& t = *static_cast<const SbFdmTables*>(pc->sb_fdm);
   switch (op->n) {
-    case 2: return sb_fdm_launch<2>(a, t, s);
-    case 3: return sb_fdm_launch<3>(a, t, s);
     case 4: return sb_fdm_launch<4>(a, t, s);
     case 5: return sb_fdm_launch<5>(a, t, s);
   }

@@ -619,9 +619,9 @@ class Preconditioner:
     def scaled_block_jacobi(cls, op, engine="tensor"):
         """For an FP32 operator with kappa_cell (no mass): z_c = H_t^-1 r_c / kappa_c
         with the shared kappa = 1 blocks H_t of the cell's boundary type.
-        engine: "tensor" (applied directly by fast diagonalisation; in solves as
-        products with the dense inverses, on the tensor cores for p = 3, 4) or "fma"
-        (the dense inverses throughout, FP32 FMA)."""
+        engine: "tensor" (p = 3, 4: applied directly by fast diagonalisation, in
+        solves as products with the dense inverses on the tensor cores) or "fma" (the
+        dense inverses throughout, FP32 FMA)."""
         h = C.c_void_p()
         eng = {"tensor": 0, "fma": 1}[engine]
         check(lib().gbfem_preconditioner_scaled_block_jacobi_create_engine(op.handle, eng, C.byref(h)))

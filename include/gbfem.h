@@ -211,12 +211,12 @@ int gbfem_preconditioner_sor_create(gbfem_operator assembled, int method, int it
  * the reference.  op must outlive pc. */
 int gbfem_preconditioner_scaled_block_jacobi_create(gbfem_operator op, gbfem_preconditioner* pc);
 /* The same with the engine chosen.  GBFEM_SB_ENGINE_TENSOR (the default of the
- * create call above): gbfem_preconditioner_apply takes H_t^{-1} in its
- * tensor-product form, by the eigenvectors of its 1-D factors (fast
- * diagonalisation, FP32 FMA); the solves take the dense inverses, for blocks of
- * 33 to 128 dofs (p = 3, 4) as products with tiles of cells of one boundary
- * type on the tcgen05 tensor cores (TF32 with the 3xTF32 split, FP32
- * accuracy), and so keep the rounding of their results.
+ * create call above): the dense inverses, for blocks of 33 to 128 dofs (p = 3,
+ * 4) as products with tiles of cells of one boundary type on the tcgen05 tensor
+ * cores (TF32 with the 3xTF32 split, FP32 accuracy) -- in the solves, which so keep
+ * the rounding of their results; gbfem_preconditioner_apply takes H_t^{-1} of
+ * p = 3, 4 in its tensor-product form, by the eigenvectors of its 1-D factors
+ * (fast diagonalisation, FP32 FMA).
  * GBFEM_SB_ENGINE_FMA: the dense inverses throughout, the tiles in FP32 FMA. */
 #define GBFEM_SB_ENGINE_TENSOR 0
 #define GBFEM_SB_ENGINE_FMA 1

@@ -58,3 +58,21 @@ def test_block_singular_up_to_rounding(gb, order):
         except gb.GbfemError as e:
             out.append(str(e))
     assert out[0] == out[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [1, 2])
+def test_low_orders_keep_the_dense_products(gb, order):
+    """p <= 2: sums of at most 27 FP32 products, which the diagonalised form's six
+    rounded contractions do not match: the dense engine's bits."""
+    cells = (11, 10, 9)
+    rng = np.random.default_rng(order)
+    op = gb.DGOperator(cells, order, precision=gb.F32,
+                       kappa_cell=gb.DeviceArray.from_numpy(np.exp(rng.uniform(-2, 2, 990)).astype(np.float32)))
+    r = gb.DeviceArray.from_numpy(rng.uniform(-1, 1, op.size).astype(np.float32))
+    out = []
+    for engine in ("tensor", "fma"):
+        z = gb.DeviceArray(op.size, gb.F32)
+        gb.Preconditioner.scaled_block_jacobi(op, engine=engine)(r, z)
+        out.append(z.numpy())
+    assert np.array_equal(*out)
