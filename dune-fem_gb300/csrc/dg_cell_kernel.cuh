@@ -10,8 +10,7 @@
 // values) plus one per face on the brick's lower boundary (80; 17.4 KB at Q1).
 // Slots are rows of 16-byte chunks, XOR-swizzled by the slot index, so lanes at
 // consecutive slots read distinct banks without padding.
-//  0. every thread loads its cell's dofs (float4 loads where the cell's block
-//     is 16-byte aligned).  Halo items, spread over the threads, load the
+//  0. every thread loads its cell's dofs (float4 loads).  Halo items, spread over the threads, load the
 //     brick's face neighbours outside it (2 (8*4 + 8*4 + 4*4) cells per 128,
 //     read through L2 -- the only traffic besides u and w) and write the
 //     trace of each one's face that touches the brick into that face's slot;
@@ -46,10 +45,8 @@ constexpr int kCellThreads = kCellBX * kCellBY * kCellBZ;
 
 template <int N>
 struct CellSlots {
-  static constexpr int N2 = N * N;
-  static constexpr int H = (N2 + 3) / 4 * 4;  // floats per half slot (v or Val | P or G), float4-aligned
-  static constexpr int Q = H / 2;             // float4 chunks in use per slot
-  static constexpr int QS = Q <= 2 ? 2 : (Q <= 4 ? 4 : 8);  // chunks per slot (a power of two)
+  static_assert(N == 2, "half a slot is one float4");
+  static constexpr int QS = 2;  // float4 chunks per slot: v or Val | P or G
   static constexpr int NX = (kCellBX + 1) * kCellBY * kCellBZ;
   static constexpr int NY = kCellBX * (kCellBY + 1) * kCellBZ;
   static constexpr int NZ = kCellBX * kCellBY * (kCellBZ + 1);
@@ -170,60 +167,38 @@ __device__ __forceinline__ void cell_boundary_flux(bool upper, const float (&vo)
   }
 }
 
-// Writes a[0..N2) and b[0..N2) into slot s (float4 stores, zero padding).
+// a and b into slot s.
 template <int N>
 __device__ __forceinline__ void cell_store_slot(float* slots, int s, const float (&a)[N * N],
                                                 const float (&b)[N * N]) {
-  constexpr int N2 = N * N, H = CellSlots<N>::H;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const float* src = h ? b : a;
-#pragma unroll
-    for (int q = 0; q < H / 4; ++q) {
-      float4 t;
-      t.x = 4 * q + 0 < N2 ? src[4 * q + 0] : 0.f;
-      t.y = 4 * q + 1 < N2 ? src[4 * q + 1] : 0.f;
-      t.z = 4 * q + 2 < N2 ? src[4 * q + 2] : 0.f;
-      t.w = 4 * q + 3 < N2 ? src[4 * q + 3] : 0.f;
-      *cell_chunk<N>(slots, s, h * (H / 4) + q) = t;
-    }
-  }
+  *cell_chunk<N>(slots, s, 0) = make_float4(a[0], a[1], a[2], a[3]);
+  *cell_chunk<N>(slots, s, 1) = make_float4(b[0], b[1], b[2], b[3]);
 }
 
 template <int N>
 __device__ __forceinline__ void cell_load_slot(float* slots, int s, float (&a)[N * N], float (&b)[N * N]) {
-  constexpr int N2 = N * N, H = CellSlots<N>::H;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float* dst = h ? b : a;
-#pragma unroll
-    for (int q = 0; q < H / 4; ++q) {
-      const float4 t = *cell_chunk<N>(slots, s, h * (H / 4) + q);
-      if (4 * q + 0 < N2) dst[4 * q + 0] = t.x;
-      if (4 * q + 1 < N2) dst[4 * q + 1] = t.y;
-      if (4 * q + 2 < N2) dst[4 * q + 2] = t.z;
-      if (4 * q + 3 < N2) dst[4 * q + 3] = t.w;
-    }
+    const float4 t = *cell_chunk<N>(slots, s, h);
+    dst[0] = t.x;
+    dst[1] = t.y;
+    dst[2] = t.z;
+    dst[3] = t.w;
   }
 }
 
 // Loads a cell's n^3 dofs into registers.
 template <int N>
 __device__ __forceinline__ void cell_load_dofs(const float* __restrict__ src, float (&x)[N * N * N]) {
-  constexpr int N3 = N * N * N;
-  if constexpr (N3 % 4 == 0) {
-    const float4* s4 = reinterpret_cast<const float4*>(src);
+  const float4* s4 = reinterpret_cast<const float4*>(src);
 #pragma unroll
-    for (int q = 0; q < N3 / 4; ++q) {
-      const float4 t = __ldg(s4 + q);
-      x[4 * q] = t.x;
-      x[4 * q + 1] = t.y;
-      x[4 * q + 2] = t.z;
-      x[4 * q + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < N3; ++e) x[e] = __ldg(src + e);
+  for (int q = 0; q < N * N * N / 4; ++q) {
+    const float4 t = __ldg(s4 + q);
+    x[4 * q] = t.x;
+    x[4 * q + 1] = t.y;
+    x[4 * q + 2] = t.z;
+    x[4 * q + 3] = t.w;
   }
 }
 
@@ -321,7 +296,6 @@ __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_c
                                                                   double* __restrict__ partial, CgScalars* sc) {
   if (DOT && !sc->active) return;
   constexpr int N2 = N * N, N3 = N2 * N;
-  using S = CellSlots<N>;
   static_assert(!(KC && ADV), "cellwise kappa without advection");
   extern __shared__ __align__(16) float slots[];
   const int tid = threadIdx.x;
@@ -433,54 +407,46 @@ __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_c
     const int s0 = cell_slot<N>(D, l[D], la, lb);      // lower face
     const int s1 = cell_slot<N>(D, l[D] + 1, la, lb);  // upper face
     const float gscale = KC ? -tabs.A2[D] * kc : 1.f;
+    float v0a[N2], g0a[N2], v1a[N2], g1a[N2];
+    cell_load_slot<N>(slots, s0, v0a, g0a);
+    cell_load_slot<N>(slots, s1, v1a, g1a);
 #pragma unroll
-    for (int q = 0; q < S::H / 4; ++q) {
-      const float4 V0 = *cell_chunk<N>(slots, s0, q);
-      const float4 G0 = *cell_chunk<N>(slots, s0, S::H / 4 + q);
-      const float4 V1 = *cell_chunk<N>(slots, s1, q);
-      const float4 G1 = *cell_chunk<N>(slots, s1, S::H / 4 + q);
-      const float v0a[4] = {V0.x, V0.y, V0.z, V0.w}, g0a[4] = {G0.x, G0.y, G0.z, G0.w};
-      const float v1a[4] = {V1.x, V1.y, V1.z, V1.w}, g1a[4] = {G1.x, G1.y, G1.z, G1.w};
+    for (int jk = 0; jk < N2; ++jk) {
+      // own view: Val_0 = -slot0, Val_1 = slot1 (G likewise)
+      const float vs = v1a[jk] - v0a[jk], vd = v1a[jk] + v0a[jk];
+      float gs = g1a[jk] - g0a[jk], gd = g1a[jk] + g0a[jk];
+      if (KC) {
+        gs *= gscale;
+        gd *= gscale;
+      }
+      float x[N];
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int jk = 4 * q + t;
-        if (jk >= N2) continue;
-        // own view: Val_0 = -slot0, Val_1 = slot1 (G likewise)
-        const float vs = v1a[t] - v0a[t], vd = v1a[t] + v0a[t];
-        float gs = g1a[t] - g0a[t], gd = g1a[t] + g0a[t];
+      for (int i = 0; i < N; ++i) x[i] = u[cell_line_off<N, D>(jk, i)];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        float& out = w[cell_line_off<N, D>(jk, i)];
+        float acc = D == 0 ? 0.f : out;
         if (KC) {
-          gs *= gscale;
-          gd *= gscale;
-        }
-        float x[N];
+          float tt = 0.f;
 #pragma unroll
-        for (int i = 0; i < N; ++i) x[i] = u[cell_line_off<N, D>(jk, i)];
+          for (int jj = 0; jj < N; ++jj)
+            if (i != 0 && jj != 0 && !((i + jj) & 1)) tt = fmaf(tabs.M[D][i * N + jj], x[jj], tt);
+          acc = fmaf(kc, tt, acc);
+          if (D == 0 && has_massK) acc = fmaf(tabs.massK, x[i], acc);
+          acc = fmaf(tabs.tr[N + i], (i & 1) ? vd : vs, acc);
+          if (i > 0) acc = fmaf(tabs.dtr[N + i], (i & 1) ? gd : gs, acc);
+        } else {
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-          float& out = w[cell_line_off<N, D>(jk, i)];
-          float acc = D == 0 ? 0.f : out;
-          if (KC) {
-            float tt = 0.f;
-#pragma unroll
-            for (int jj = 0; jj < N; ++jj)
-              if (i != 0 && jj != 0 && !((i + jj) & 1)) tt = fmaf(tabs.M[D][i * N + jj], x[jj], tt);
-            acc = fmaf(kc, tt, acc);
-            if (D == 0 && has_massK) acc = fmaf(tabs.massK, x[i], acc);
-            acc = fmaf(tabs.tr[N + i], (i & 1) ? vd : vs, acc);
-            if (i > 0) acc = fmaf(tabs.dtr[N + i], (i & 1) ? gd : gs, acc);
-          } else {
-#pragma unroll
-            for (int jj = 0; jj < N; ++jj) {
-              const bool mass00 = D == 0 && i == 0 && jj == 0 && has_mass;
-              const bool k1 = i != 0 && jj != 0 && !((i + jj) & 1);
-              const bool d1 = jj < i && ((i + jj) & 1);
-              if (k1 || mass00 || (ADV && d1)) acc = fmaf(tabs.M[D][i * N + jj], x[jj], acc);
-            }
-            acc = fmaf(tabs.etr[D][i], (i & 1) ? vd : vs, acc);
-            if (i > 0) acc = fmaf(tabs.edtr[D][i], (i & 1) ? gd : gs, acc);
+          for (int jj = 0; jj < N; ++jj) {
+            const bool mass00 = D == 0 && i == 0 && jj == 0 && has_mass;
+            const bool k1 = i != 0 && jj != 0 && !((i + jj) & 1);
+            const bool d1 = jj < i && ((i + jj) & 1);
+            if (k1 || mass00 || (ADV && d1)) acc = fmaf(tabs.M[D][i * N + jj], x[jj], acc);
           }
-          out = acc;
+          acc = fmaf(tabs.etr[D][i], (i & 1) ? vd : vs, acc);
+          if (i > 0) acc = fmaf(tabs.edtr[D][i], (i & 1) ? gd : gs, acc);
         }
+        out = acc;
       }
     }
   };
@@ -492,14 +458,9 @@ __global__ void __launch_bounds__(kCellThreads, 3) dg_cell_kernel(const __grid_c
 
     // ---- 4. store ----------------------------------------------------------------
     float* dst = args.w + cell * N3;
-    if constexpr (N3 % 4 == 0) {
-      float4* d4 = reinterpret_cast<float4*>(dst);
+    float4* d4 = reinterpret_cast<float4*>(dst);
 #pragma unroll
-      for (int q = 0; q < N3 / 4; ++q) __stcs(d4 + q, make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]));
-    } else {
-#pragma unroll
-      for (int q = 0; q < N3; ++q) __stcs(dst + q, w[q]);
-    }
+    for (int q = 0; q < N3 / 4; ++q) __stcs(d4 + q, make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]));
     if (DOT) {
 #pragma unroll
       for (int q = 0; q < N3; ++q) acc.add(u[q], w[q]);

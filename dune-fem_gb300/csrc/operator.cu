@@ -521,14 +521,14 @@ static int host_pipe(gbfem_operator_s* op, int nchunks, HostPipe** out) {
 
 // Host-buffer apply of a DG operator, pipelined over slabs of whole z-planes
 // (a slab is a contiguous range of cells and dofs): the host-to-device copy
-// of slab k+1, the trace pass of slab k+1, the apply of slab k and the
-// device-to-host copy of slab k-1 run at the same time on four streams.  The
-// apply of a slab needs its z-neighbours' data (their traces for the
-// closed-form kernel, their dofs for the quadrature kernel), so it is issued
-// once the next slab's traces exist (or it has arrived); with periodic z,
-// slab 0 also needs the last slab and is applied last.  Each cell is computed
-// by the same kernel code as the one-shot apply, so the result is bitwise the
-// same.
+// of slab k+1, the apply of slab k and the device-to-host copy of slab k-1 run
+// at the same time on three streams; the two-kernel closed form (FP32, and FP64
+// operators that fixed point does not take) has the trace pass of slab k+1 on a
+// fourth.  The apply of a slab needs its z-neighbours' data (their dofs, or
+// their traces in that form), so it is issued once the next slab has arrived
+// (its traces exist); with periodic z, slab 0 also needs the last slab and is
+// applied last.  Each cell is computed by the same kernel code as the one-shot
+// apply (FP32: as GBFEM_ALGO_TRACE_PASS), so the result is bitwise the same.
 
 // The device address of page-locked (registered or cudaHostAlloc'ed) host
 // memory, or nullptr for anything else.  Only such memory is ever read or
@@ -543,13 +543,13 @@ static void* mapped_device_pointer(const void* host) {
   return a.devicePointer;
 }
 
-// Host-buffer apply of the closed-form kernel on page-locked buffers: the
-// trace pass reads u straight from host memory over NVLink-C2C (and leaves a
-// device copy for the main kernel), the main kernel writes w straight to host
-// memory.  Slabs of z-planes as in the copy pipeline: traces of slab k on one
-// stream, the apply of slab k-1 on another once slab k's traces exist, so the
-// C2C reads overlap the FP64 work.  Same kernels and arithmetic as the
-// device apply.
+// Host-buffer apply of the closed form on page-locked buffers: the first phase
+// reads u straight from host memory over NVLink-C2C and leaves a device copy
+// for the apply (the FP64 fixed-point form only copies; the two-kernel form
+// makes its traces on the way), and the apply writes w straight to host memory.
+// Slabs of z-planes as in the copy pipeline: phase one of slab k on one stream,
+// the apply of slab k-1 on another once slab k is there, so the C2C reads
+// overlap the arithmetic.  Same kernels and arithmetic as the device apply.
 static int dg_apply_host_mapped(gbfem_operator_s* op, const void* du, void* dw) {
   const int nz = op->dg.grid.cells[2];
   const long long plane = (long long)op->dg.grid.cells[0] * op->dg.grid.cells[1];
