@@ -3,8 +3,8 @@
 // contractions as dg_apply_kernel (dg_kernel.cuh), which is bound by the FP64
 // pipe (270 multiply-adds per dof at Q3, 0.5 clocks each on an SM).
 //
-// What bounds it: integer issue and the barriers between the contractions (2.1
-// instructions a clock and SM), about 3600 instructions per dof at Q3 in place of 135
+// What bounds it: integer issue and the barriers between the contractions (2.3
+// instructions a clock and SM), about 3500 instructions per dof at Q3 in place of 135
 // clocks of FP64 pipe.  Measured (GB300), dg_apply_kernel before, this after:
 // 45 x 38 x 33 Q3 2152 -> 571 us.
 //

@@ -1,4 +1,6 @@
-// Scaled shared-block Jacobi on the 5th-generation tensor cores (tcgen05).
+// Scaled shared-block Jacobi on the 5th-generation tensor cores (tcgen05): the form
+// the solves take for p = 3 and 4 (a direct apply goes by fast diagonalisation,
+// sb_fdm.cu, which is faster but rounds differently).
 //
 // The preconditioner z_c = H_t(c)^-1 r_c / kappa_c of a cellwise-kappa DG
 // operator (solver.cu) applied to tiles of up to 32 cells of one boundary

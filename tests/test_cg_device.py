@@ -87,3 +87,31 @@ def test_q1_general_loop(gb, cells):
         assert rc == 0 and info.converged
         out.append((info.iterations, info.residual, u.numpy().tobytes()))
     assert out[0] == out[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [3, 4])
+@pytest.mark.parametrize("cells,periodic", [((5, 4, 3), (0, 0, 0)), ((20, 18, 16), (0, 1, 1)), ((40, 36, 32), (0, 0, 1))])
+def test_solves_take_the_tensor_core_tiles(gb, order, cells, periodic):
+    """One CG step, x = alpha P b, with the dense products on the tensor cores and in
+    FP32 FMA: type changes per CTA, and on the largest grid several full tiles per CTA
+    through the pipeline.  FP32 sums of up to 125 terms: the 2e-5 of the direct
+    apply's test."""
+    rng = np.random.default_rng(order)
+    op = gb.DGOperator(cells, order, precision=gb.F32, periodic=periodic,
+                       kappa_cell=gb.DeviceArray.from_numpy(rng.uniform(0.5, 2, np.prod(cells)).astype(np.float32)))
+    f, out = gb.DeviceArray.from_numpy(rng.uniform(-1, 1, op.size).astype(np.float32)), {}
+    for engine in ("tensor", "fma"):
+        pc = gb.Preconditioner.scaled_block_jacobi(op, engine=engine)
+        inv = gb.KrylovInverseOperator("cg", tolerance=1e-30, max_iterations=1)
+        inv.bind(op, pc)
+        for _ in range(2):
+            u = gb.DeviceArray(op.size, gb.F32)
+            u.clear()
+            inv(f, u)
+            assert pc.status() == 0
+            if engine in out:  # twice the same bits
+                assert np.array_equal(out[engine].view(np.uint32), u.numpy().view(np.uint32))
+            out[engine] = u.numpy()
+    assert np.max(np.abs(out["tensor"] - out["fma"])) <= 2e-5 * np.max(np.abs(out["fma"]))
+    assert not np.array_equal(out["tensor"], out["fma"])
