@@ -247,9 +247,11 @@ static void sb_eigen(int n, double (&a)[kDgMaxN][kDgMaxN], double (&V)[kDgMaxN][
   }
 }
 
-// The tables, in pc->sb_fdm; left null for p <= 2 (above) and where a block is singular to FP32 rounding (one
-// cell without a boundary term: the division gives infinities, the dense inverse of
-// the rounded block does not).
+// The tables, in pc->sb_fdm; left null for p <= 2 (above) and where a block is not
+// positive definite: a penalty too small, whose eigenvalues' sums cancel (penalty 0,
+// Q3: error 1e-5), or one cell without a boundary term, where the division gives
+// infinities and the dense inverse of the rounded block does not.  Positive definite
+// blocks keep 2e-7 up to condition numbers of 1e6.
 int sb_fdm_setup(gbfem_preconditioner_s* pc) {
   const gbfem_operator_s* op = pc->sor_op;
   const gbfem_dg_desc& d = op->dg;
@@ -299,11 +301,11 @@ int sb_fdm_setup(gbfem_preconditioner_s* pc) {
     if (!occurs(0, ty[0]) || !occurs(1, ty[1]) || !occurs(2, ty[2])) continue;
     float least = INFINITY, most = 0.f;
     for (int l = 0; l < n * n * n; ++l) {
-      const float v = fabsf(t->L[0][ty[0]][l / (n * n)] + t->L[1][ty[1]][(l / n) % n] + t->L[2][ty[2]][l % n]);
+      const float v = t->L[0][ty[0]][l / (n * n)] + t->L[1][ty[1]][(l / n) % n] + t->L[2][ty[2]][l % n];
       least = fminf(least, v);
       most = fmaxf(most, v);
     }
-    regular = regular && least > 1e-6f * most;
+    regular = regular && least > 1e-7f * most;
   }
   if (regular) pc->sb_fdm = t;
   else delete t;

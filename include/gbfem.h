@@ -214,8 +214,8 @@ int gbfem_preconditioner_scaled_block_jacobi_create(gbfem_operator op, gbfem_pre
  * create call above): the dense inverses, for blocks of 33 to 128 dofs (p = 3,
  * 4) as products with tiles of cells of one boundary type on the tcgen05 tensor
  * cores (TF32 with the 3xTF32 split, FP32 accuracy) -- in the solves, which so keep
- * the rounding of their results; gbfem_preconditioner_apply takes H_t^{-1} of
- * p = 3, 4 in its tensor-product form, by the eigenvectors of its 1-D factors
+ * the rounding of their results; gbfem_preconditioner_apply takes positive definite
+ * H_t^{-1} of p = 3, 4 in its tensor-product form, by the eigenvectors of its 1-D factors
  * (fast diagonalisation, FP32 FMA).
  * GBFEM_SB_ENGINE_FMA: the dense inverses throughout, the tiles in FP32 FMA. */
 #define GBFEM_SB_ENGINE_TENSOR 0

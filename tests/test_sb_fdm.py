@@ -76,3 +76,33 @@ def test_low_orders_keep_the_dense_products(gb, order):
         gb.Preconditioner.scaled_block_jacobi(op, engine=engine)(r, z)
         out.append(z.numpy())
     assert np.array_equal(*out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("order", [3, 4])
+@pytest.mark.parametrize("kw,dense", [(dict(), False), (dict(penalty=0.3), True), (dict(penalty=1.0), True),
+                                      (dict(penalty=1.0, weak_dirichlet=False, upper=(1.0, 0.5, 2.0)), True)])
+def test_indefinite_blocks_take_the_dense_products(gb, order, kw, dense):
+    """A small penalty: the sums of the 1-D eigenvalues cancel, and the division would
+    amplify their rounding.  The direct apply z = P r is then the solves': the first
+    CG iterate is alpha z, rounded once, for one FP32 alpha."""
+    cells, n = (6, 7, 3), 126 * (order + 1) ** 3
+    rng = np.random.default_rng(order)
+    op = gb.DGOperator(cells, order, precision=gb.F32,
+                       kappa_cell=gb.DeviceArray.from_numpy(np.exp(rng.uniform(-1, 1, 126)).astype(np.float32)), **kw)
+    pc = gb.Preconditioner.scaled_block_jacobi(op)
+    inv = gb.KrylovInverseOperator("cg", tolerance=1e-30, max_iterations=1)
+    inv.bind(op, pc)
+    for _ in range(40):  # <r, P r> > 0, or there is no step
+        r, z, x = gb.DeviceArray.from_numpy(rng.uniform(-1, 1, n).astype(np.float32)), *(gb.DeviceArray(n, gb.F32) for _ in "zx")
+        x.clear()
+        inv(r, x)
+        if x.numpy().any():
+            break
+    pc(r, z)
+    x, z = x.numpy(), z.numpy()
+    j = np.argmax(np.abs(x))
+    near = [np.float32(x[j] / z[j])]
+    for way in (np.float32(-np.inf), np.float32(np.inf)):
+        near += [np.nextafter(near[0], way), np.nextafter(np.nextafter(near[0], way), way)]
+    assert x.any() and any(np.array_equal(a * z, x) for a in near) == dense
